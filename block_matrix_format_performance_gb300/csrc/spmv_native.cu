@@ -21,7 +21,7 @@
 //    Q = 32/bs, then a shuffle tree sums over q.
 //  * bcsr_row_kernel (bs > 32): one thread per scalar row.
 //  * csr_subwarp_kernel: G lanes per row, strided over its entries
-//    (the bs = 1 case and plain CSR).
+//    (the bs = 1 case and plain CSR); the warp together for long rows.
 //
 // Values are loaded with the streaming (evict-first) hint, x through the
 // read-only path. No tensor cores: a single-vector product has no reuse of A
@@ -144,16 +144,35 @@ __global__ void __launch_bounds__ (kThreads)
   y[idx] = acc;
 }
 
+// G lanes per row, with G a fraction of the average row: a row's sum costs
+// log2 G warp-wide FP64 adds beside its multiply-adds, and GB300's FP64 pipe
+// charges each of them in full. A row far above the average would then run
+// long on its few lanes, so the warp takes such rows together afterwards.
 template <typename T, int G>
 __global__ void __launch_bounds__ (kThreads)
   csr_subwarp_kernel (int n_rows, const int *__restrict__ row_ptr, const int *__restrict__ cols,
                       const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
 {
-  const int64_t group = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const int64_t n_groups = (int64_t) gridDim.x * blockDim.x / G;
+  constexpr int kLongRow = 16 * G + 48;
+  const int64_t row = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / G;
   core::NoEpilogue epi;
-  for (int64_t row = group; row < n_rows; row += n_groups)
-    core::csr_row<T, G> ((int) row, row_ptr, cols, vals, x, y, epi);
+  bool wide = false;
+  if (row < n_rows)
+    {
+      wide = G < 32 && __ldg (row_ptr + row + 1) - __ldg (row_ptr + row) > kLongRow;
+      if (!wide)
+        core::csr_row<T, G> ((int) row, row_ptr, cols, vals, x, y, epi);
+    }
+  if constexpr (G < 32)
+    {
+      unsigned left = __ballot_sync (0xffffffffu, wide && (threadIdx.x & (G - 1)) == 0);
+      while (left)
+        {
+          const int src = __ffs (left) - 1;
+          left &= left - 1;
+          core::csr_row<T, 32> ((int) __shfl_sync (0xffffffffu, (int) row, src), row_ptr, cols, vals, x, y, epi);
+        }
+    }
 }
 
 // ---------------------------------------------------------------- dispatch
@@ -224,10 +243,16 @@ int launch_csr (int n, int g, const int *rp, const int *c, const T *v, const T *
     }
 }
 
+// Lanes per CSR row. Measured with the matrices read from HBM, us for 1, 2, 4,
+// 8, 16 and 32 lanes: the 1000x250 elasticity operator (18 entries a row) in
+// FP64 77 / 42 / 32 / 48 / 106 / 215; four million entries in rows of 2.5 on
+// average 19 / 27 / 52 / 87 / 207 / -, 7.5: 19 / 21 / 27 / 46 / 79 / -,
+// 11.5: 22 / 20 / 23 / 32 / 63 / -, 26: 23 / 21 / 20 / 23 / 34 / -,
+// 39: 30 / 23 / 20 / 21 / 27 / -, 64: 44 / 26 / 22 / 20 / 23 / -.
 inline int csr_default_lanes (double avg_nnz_per_row)
 {
   int g = 1;
-  while (g < 32 && g < avg_nnz_per_row)
+  while (g < 32 && 7 * g < avg_nnz_per_row)
     g <<= 1;
   return g;
 }
@@ -304,14 +329,7 @@ int native_bcsr_typed (int nbr, int bs, int64_t nnzb, const int *rp, const int *
 int native_default_lanes (int dtype, int bs, double avg_blocks_per_row)
 {
   if (bs == 1)
-    {
-      // A few lanes per CSR row: the autotuner picked 1-2 on GB300 for eight
-      // entries per row.
-      int g = 1;
-      while (g < 32 && 4 * g < avg_blocks_per_row)
-        g <<= 1;
-      return g;
-    }
+    return csr_default_lanes (avg_blocks_per_row);
   if (!flat_bs (bs))
     return 32;
   // The choices bmfp_matrix_autotune made on GB300 for the block-size sweep

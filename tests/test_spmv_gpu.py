@@ -169,6 +169,34 @@ def test_csr_variant_parity(lib, orc, cuda, variant, bs, dtype):
     assert np.all(np.abs(y[:n] - y_ref) <= spmv_tolerance(orc, crp, cc, cv, x, dtype))
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("lanes", [0, 1, 2, 4, 8, 16, 32])
+def test_csr_rows_far_above_the_average(lib, orc, cuda, lanes, dtype):
+    """Rows on both sides of the length from which a whole warp takes a row
+    (16 G + 48 entries for G lanes), several in one warp, the last row among
+    them, on a row count that is no multiple of the rows per warp."""
+    import torch
+    rng = np.random.default_rng(lanes)
+    g = lanes or 2
+    counts = rng.integers(0, 6, 1003)
+    edge = 16 * g + 48
+    for i, k in ((0, edge), (1, edge + 1), (2, 700), (3, edge + 2), (40, 1500), (41, 2), (500, edge - 1), (1002, 900)):
+        counts[i] = k
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    c = np.concatenate([np.sort(rng.choice(2000, size=k, replace=False)) for k in counts]).astype(np.int32)
+    v = rng.uniform(-1, 1, c.size).astype(dtype)
+    x = rng.uniform(-1, 1, 2000).astype(dtype)
+    d_y = torch.full((1003 + GUARD,), float("nan"), dtype=torch.float64 if dtype == np.float64 else torch.float32,
+                     device="cuda")
+    if lanes == 0:
+        bm.csr_spmv(bm.CSR_NATIVE, dev(rp), dev(c), dev(v), dev(x), d_y)
+    else:
+        bm.bcsr_spmv_native(dev(rp), dev(c), dev(v), dev(x), d_y, 1, lanes=lanes)
+    y = d_y.cpu().numpy()
+    assert np.isnan(y[1003:]).all()
+    assert np.all(np.abs(y[:1003] - orc.csr_spmv(rp, c, v, x)) <= spmv_tolerance(orc, rp, c, v, x, dtype))
+
+
 def test_empty_and_zero_block_matrices(lib, orc, cuda):
     import torch
     # no block rows at all: a valid no-op
