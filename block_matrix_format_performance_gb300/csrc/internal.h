@@ -41,6 +41,11 @@ int spmv_native_bcsr (int dtype, int n_block_rows, int bs, int64_t nnzb, const i
                       cudaStream_t stream);
 int spmv_native_csr (int dtype, int n_rows, int64_t nnz, const int *row_ptr, const int *cols,
                      const void *vals, const void *x, void *y, int lanes, cudaStream_t stream);
+// The same product for 3 <= bs <= 32 by row tiles staged in shared memory (vals
+// and cols 16-byte aligned); *took is false, and nothing is launched, where
+// the matrix has too few tiles to fill the GPU.
+int spmv_tile (int dtype, int n_block_rows, int bs, int64_t nnzb, const int *row_ptr, const int *cols,
+               const void *vals, const void *x, void *y, bool *took, cudaStream_t stream);
 int spmv_reference_variant (int dtype, int variant, int n_rows, int n_cols, int bs, int64_t nnz,
                             const int *row_ptr, const int *cols, const void *vals, const void *x,
                             void *y, cudaStream_t stream);

@@ -16,7 +16,9 @@
 //    and a fixed set of rows per phase (chunk < block). Partial row sums are
 //    combined with xor-shuffles over exactly the lane bits that vary the
 //    column, so the reduction costs log2 steps and no shared memory.
-//  * bcsr_tpr_kernel (any bs <= 32, e.g. 3 for frame elements): a warp owns
+//  * row tiles (spmv_tile.cu: bs <= 32 that is no power of two, e.g. 3 for
+//    frame elements, from a few hundred tiles up).
+//  * bcsr_tpr_kernel (any bs <= 32, small or misaligned): a warp owns
 //    a block row, lane (q, r) takes scalar row r of blocks q, q+Q, ... with
 //    Q = 32/bs, then a shuffle tree sums over q.
 //  * bcsr_row_kernel (bs > 32): one thread per scalar row.
@@ -309,6 +311,16 @@ int native_bcsr_typed (int nbr, int bs, int64_t nnzb, const int *rp, const int *
     }
   if (bs <= 32)
     {
+      // Row tiles, except at bs 9 in FP32, where the warp per block row is
+      // level with them (35 against 35 us on rows of 0-15 blocks).
+      const bool staged = ((reinterpret_cast<uintptr_t> (v) | reinterpret_cast<uintptr_t> (c)) & 15u) == 0;
+      if (!flat_bs (bs) && staged && !(bs == 9 && sizeof (T) == 4))
+        {
+          bool took = false;
+          const int st = spmv_tile (dtype, nbr, bs, nnzb, rp, c, v, x, y, &took, s);
+          if (st != BMFP_SUCCESS || took)
+            return st;
+        }
       const int64_t threads = (int64_t) nbr * 32;
       const unsigned grid = (unsigned) ((threads + kThreads - 1) / kThreads);
       if (bs == 3)

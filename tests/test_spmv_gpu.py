@@ -197,6 +197,50 @@ def test_csr_rows_far_above_the_average(lib, orc, cuda, lanes, dtype):
     assert np.all(np.abs(y[:1003] - orc.csr_spmv(rp, c, v, x)) <= spmv_tolerance(orc, rp, c, v, x, dtype))
 
 
+def tiled_bcsr(bs, dtype, seed, kind):
+    """A BCSR matrix with enough blocks for the row-tile kernel. kind: rows of
+    0-15 blocks; mostly empty rows; rows far longer than a tile among them."""
+    rng = np.random.default_rng(seed)
+    slots = 128 // bs
+    per_tile = max(1, round((20 if bs <= 5 else 24) * 1024 / ((bs * bs * np.dtype(dtype).itemsize + 4) * slots))) * slots
+    nbr = int(per_tile * 520 / 7.5) + 3 if kind != "sparse" else int(per_tile * 520 / 0.5) + 3
+    nbr = min(nbr, 1024 * 460 + 5)
+    if kind == "sparse":
+        counts = (rng.random(nbr) < 0.2).astype(int)
+    else:
+        counts = rng.integers(0, 16, nbr)
+        if kind == "long":
+            counts[[0, 7, nbr - 1]] = [3 * per_tile, per_tile, 2 * per_tile + 1]
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    nbc = nbr
+    cols = rng.integers(0, nbc, int(rp[-1])).astype(np.int32)
+    vals = rng.uniform(-1, 1, int(rp[-1]) * bs * bs).astype(dtype)
+    return rp, cols, vals, nbc
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("kind", ["uneven", "sparse", "long"])
+@pytest.mark.parametrize("bs", [3, 5, 6, 12, 13, 17, 22, 31])
+def test_row_tiles(lib, orc, cuda, bs, kind, dtype):
+    """Block sizes with a kernel of their own and without, both x alignments
+    (an odd offset takes scalar loads of x), rows cut by tiles' pieces."""
+    if bs > 13 and kind == "sparse":
+        pytest.skip("the small block sizes cover mostly empty rows")
+    import torch
+    rp, c, v, nbc = tiled_bcsr(bs, dtype, bs, kind)
+    n = (rp.size - 1) * bs
+    crp, cc, cv = orc.bcsr_to_csr(rp, c, v, bs)
+    for off in (0, 1) if kind == "uneven" else (0,):
+        xf = np.random.default_rng(off).uniform(-1, 1, nbc * bs + off).astype(dtype)
+        d_x = dev(xf)[off:]
+        d_y = torch.full((n + GUARD,), float("nan"), dtype=d_x.dtype, device="cuda")
+        bm.bcsr_spmv(bm.BCSR_NATIVE, dev(rp), dev(c), dev(v), d_x, d_y, bs, nbc)
+        y = d_y.cpu().numpy()
+        assert np.isnan(y[n:]).all()
+        tol = spmv_tolerance(orc, crp, cc, cv, xf[off:], dtype)
+        assert np.all(np.abs(y[:n] - orc.bcsr_spmv(rp, c, v, bs, xf[off:])) <= tol)
+
+
 def test_empty_and_zero_block_matrices(lib, orc, cuda):
     import torch
     # no block rows at all: a valid no-op
