@@ -91,14 +91,42 @@ template <typename T> struct Args
   double *part;
   int grid;
   DevState *st;
+  // Sliced copy of a bs = 2 matrix (SellOp), or null.
+  const int *soff, *scols;
+  const T *svals;
+  int nslices;
 };
 
+// Sum over a warp, the same on every lane: each value's mantissa shifted to
+// the largest exponent of the warp (five guard bits: more than the FP64 adds
+// of a butterfly keep), the integers added exactly in three limbs by redux,
+// one rounding at the end. A butterfly's five dependent warp-wide FP64 adds
+// take about 500 cycles and keep GB300's narrow FP64 pipe busy throughout;
+// this takes about 150 on the integer pipes. Zeros, subnormals, infinities and
+// NaN go to the butterfly.
 __device__ __forceinline__ double warp_sum (double v)
 {
+  constexpr unsigned kAll = 0xffffffffu;
+  const long long bits = __double_as_longlong (v);
+  const int ex = (int) ((bits >> 52) & 0x7ff);
+  const int top = (int) __reduce_max_sync (kAll, (unsigned) ex);
+  if (top < 64 || top > 2047 - 64)
+    {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-    v += __shfl_xor_sync (0xffffffffu, v, off);
-  return v;
+      for (int off = 16; off > 0; off >>= 1)
+        v += __shfl_xor_sync (kAll, v, off);
+      return v;
+    }
+  const int d = top - ex;
+  long long m = ex ? ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 5 : 0;
+  m = d < 58 ? (m + ((1ll << d) >> 1)) >> d : 0;
+  if (bits < 0)
+    m = -m;
+  const unsigned lo = __reduce_add_sync (kAll, (unsigned) (m & 0xfffff));
+  const unsigned mid = __reduce_add_sync (kAll, (unsigned) ((m >> 20) & 0xfffff));
+  const int hi = __reduce_add_sync (kAll, (int) (m >> 40));
+  const long long sum = ((long long) hi << 40) + ((long long) mid << 20) + lo;
+  return (double) sum * __longlong_as_double ((long long) (top - 57) << 52);
 }
 
 // done and rep_now in one load. Both are written by earlier kernels (done
@@ -113,9 +141,8 @@ __device__ __forceinline__ bool is_done (const DevState *st) { return flags (st)
 
 // Sum the grid partials of NK kinds in a fixed order, broadcast to the CTA.
 // Every thread loads its share of the partials at once (the grid is a few
-// CTAs per SM, so a handful of loads each), then warps and the warps' totals
-// reduce by butterflies: a few memory round trips instead of one per 32
-// partials, on the path every phase waits for.
+// CTAs per SM, so a handful of loads each), then the warps sum, and warp k
+// sums the warps' totals of kind k.
 template <int NK>
 __device__ __forceinline__ void sum_parts (const double *part, int grid, const int (&ks)[NK],
                                            double (&out)[NK])
@@ -141,14 +168,12 @@ __device__ __forceinline__ void sum_parts (const double *part, int grid, const i
         sh_w[k][w] = s;
     }
   __syncthreads ();
-  if (w == 0)
-#pragma unroll
-    for (int k = 0; k < NK; k++)
-      {
-        const double a = warp_sum (lane < kWarps ? sh_w[k][lane] : 0.0);
-        if (lane == 0)
-          sh[k] = a;
-      }
+  if (w < NK)
+    {
+      const double a = warp_sum (lane < kWarps ? sh_w[w][lane] : 0.0);
+      if (lane == 0)
+        sh[w] = a;
+    }
   __syncthreads ();
 #pragma unroll
   for (int k = 0; k < NK; k++)
@@ -177,36 +202,28 @@ __device__ __forceinline__ bool arrive_last (DevState *st, int grid)
   return sh_last != 0;
 }
 
-// Reduce per-thread values over the CTA (fixed order) into part[k][blockIdx]:
-// a tree through shared memory (128, 64, 32 threads add pairs) and one warp
-// butterfly for the last 32. Each warp-wide FP64 add costs GB300's narrow
-// FP64 pipe the same whatever the number of useful lanes: the tree takes
-// 12 warp adds per value and CTA, a butterfly in every warp took 45.
+// Reduce per-thread values over the CTA into part[k][blockIdx]: warps, then
+// warp k over the warps' totals of kind k.
 template <int NK>
 __device__ __forceinline__ void store_parts (double (&v)[NK], double *part, int grid,
                                              const int (&ks)[NK])
 {
-  __shared__ double sh[NK][kThreads];
-  const int t = threadIdx.x;
+  __shared__ double sh[NK][kWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < NK; k++)
-    sh[k][t] = v[k];
+    {
+      const double a = warp_sum (v[k]);
+      if (lane == 0)
+        sh[k][w] = a;
+    }
   __syncthreads ();
 #pragma unroll
-  for (int h = kThreads / 2; h >= 32; h >>= 1)
-    {
-      if (t < h)
-#pragma unroll
-        for (int k = 0; k < NK; k++)
-          sh[k][t] += sh[k][t + h];
-      __syncthreads ();
-    }
-  if (t < 32)
-#pragma unroll
-    for (int k = 0; k < NK; k++)
+  for (int k = 0; k < NK; k++)
+    if (w == k)
       {
-        const double a = warp_sum (sh[k][t]);
-        if (t == 0)
+        const double a = warp_sum (lane < kWarps ? sh[k][lane] : 0.0);
+        if (lane == 0)
           part[ks[k] * grid + blockIdx.x] = a;
       }
 }
@@ -228,6 +245,200 @@ template <typename T, int BS, int G, class XL = dev::XNc> struct FlatOp
       core::flat_row<T, BS, G, 4, XL> ((int) row, a.rp, a.cols, a.vals, x, y, e);
   }
 };
+
+// Scalar rows per slice of the sliced matrix: one warp, one row per lane.
+constexpr int kSlice = 32;
+
+// bs = 2 on the sliced copy: step k of a slice holds line r of the k-th block
+// of each of its 32 scalar rows side by side, so a warp reads 512 (FP32: 256)
+// consecutive bytes per step where the row-by-row walk of the block rows
+// touched 16 lines, and every lane runs the same number of steps. Three
+// steps' x in flight and the next three steps' values and columns behind
+// them: the walk is bound by latency otherwise. Rows are padded to the
+// slice's longest with zero blocks on a column the row already reads.
+// 2000x500 Q4 grid, FP64, phases 2 and 4 by block rows and by slices: 84.5 and
+// 88.4 us -> 72.8 and 81.1 us (FP64 pipe 74 % -> 82 % busy, its work alone 61
+// and 64 us).
+template <typename T, class XL = dev::XNc> struct SellOp
+{
+  static constexpr int U = 3;
+  struct Step
+  {
+    T v0, v1;
+    int c;
+  };
+  __device__ static __forceinline__ Step load (const T *v, const int *c, int k)
+  {
+    Step s;
+    if constexpr (sizeof (T) == 8)
+      {
+        const double2 t = __ldcs (reinterpret_cast<const double2 *> (v) + (size_t) k * kSlice);
+        s.v0 = t.x;
+        s.v1 = t.y;
+      }
+    else
+      {
+        const float2 t = __ldcs (reinterpret_cast<const float2 *> (v) + (size_t) k * kSlice);
+        s.v0 = t.x;
+        s.v1 = t.y;
+      }
+    s.c = __ldg (c + (size_t) k * (kSlice / 2));
+    return s;
+  }
+  template <class Epi>
+  __device__ static void run (const Args<T> &a, const T *x, T *y, Epi &e)
+  {
+    const int lane = threadIdx.x & 31;
+    const int nw = (int) (gridDim.x * blockDim.x / kSlice);
+    int slice = (int) ((blockIdx.x * blockDim.x + threadIdx.x) / kSlice);
+    if (slice >= a.nslices)
+      return;
+    int beg = __ldg (a.soff + slice), end = __ldg (a.soff + slice + 1);
+    for (;;)
+      {
+        const int next = slice + nw;
+        int nbeg = 0, nend = 0;
+        if (next < a.nslices)
+          {
+            nbeg = __ldg (a.soff + next);
+            nend = __ldg (a.soff + next + 1);
+          }
+        const int64_t i = (int64_t) slice * kSlice + lane;
+        if (i < a.n)
+          e.pre (i);
+        const T *v = a.svals + ((size_t) beg * kSlice + lane) * 2;
+        const int *c = a.scols + (size_t) beg * (kSlice / 2) + lane / 2;
+        const int n = end - beg;
+        T acc = 0;
+        int k = 0;
+        if (n >= U)
+          {
+            Step s[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+              s[u] = load (v, c, u);
+            for (; k + 2 * U <= n; k += U)
+              {
+                Step t[U];
+                T x0[U], x1[U];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                  XL::ld2 (x + (size_t) s[u].c * 2, x0[u], x1[u]);
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                  t[u] = load (v, c, k + U + u);
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                  {
+                    acc = fma (s[u].v0, x0[u], acc);
+                    acc = fma (s[u].v1, x1[u], acc);
+                  }
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                  s[u] = t[u];
+              }
+            T x0[U], x1[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+              XL::ld2 (x + (size_t) s[u].c * 2, x0[u], x1[u]);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+              {
+                acc = fma (s[u].v0, x0[u], acc);
+                acc = fma (s[u].v1, x1[u], acc);
+              }
+            k += U;
+          }
+        for (; k < n; k++)
+          {
+            const Step s = load (v, c, k);
+            T x0, x1;
+            XL::ld2 (x + (size_t) s.c * 2, x0, x1);
+            acc = fma (s.v0, x0, acc);
+            acc = fma (s.v1, x1, acc);
+          }
+        if (i < a.n)
+          {
+            y[i] = acc;
+            e.now (i, acc);
+          }
+        if (next >= a.nslices)
+          break;
+        slice = next;
+        beg = nbeg;
+        end = nend;
+      }
+  }
+};
+
+// The sliced copy's layout: slice widths (its longest row, in blocks), their
+// running sum by one CTA (off[nslices] the total), and the fill.
+__global__ void sell_width_kernel (int nbr, const int *rp, int nslices, int *width)
+{
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nslices)
+    return;
+  const int r1 = min (nbr, (s + 1) * (kSlice / 2));
+  int w = 0;
+  for (int r = s * (kSlice / 2); r < r1; r++)
+    w = max (w, rp[r + 1] - rp[r]);
+  width[s] = w;
+}
+
+__global__ void __launch_bounds__ (1024) sell_scan_kernel (int nslices, const int *width, int *off,
+                                                           unsigned long long *total)
+{
+  __shared__ unsigned long long sh[1024];
+  const int per = (nslices + 1023) / 1024;
+  const int64_t s0 = min ((int64_t) nslices, (int64_t) threadIdx.x * per), s1 = min ((int64_t) nslices, s0 + per);
+  unsigned long long sum = 0;
+  for (int64_t s = s0; s < s1; s++)
+    sum += (unsigned) width[s];
+  sh[threadIdx.x] = sum;
+  __syncthreads ();
+  for (int h = 1; h < 1024; h <<= 1)
+    {
+      const unsigned long long v = (int) threadIdx.x >= h ? sh[threadIdx.x - h] : 0;
+      __syncthreads ();
+      sh[threadIdx.x] += v;
+      __syncthreads ();
+    }
+  unsigned long long at = sh[threadIdx.x] - sum;
+  for (int64_t s = s0; s < s1; s++)
+    {
+      off[s] = (int) at;
+      at += (unsigned) width[s];
+    }
+  if (threadIdx.x == 1023)
+    {
+      off[nslices] = (int) sh[1023];
+      *total = sh[1023];
+    }
+}
+
+template <typename T>
+__global__ void sell_fill_kernel (int nbr, const int *rp, const int *cols, const T *vals, int nslices, const int *off,
+                                  int *scols, T *svals)
+{
+  const int lane = threadIdx.x & 31;
+  const int nw = (int) (gridDim.x * blockDim.x / 32);
+  for (int s = (int) ((blockIdx.x * blockDim.x + threadIdx.x) / 32); s < nslices; s += nw)
+    {
+      const int row = s * (kSlice / 2) + lane / 2;
+      const int beg = row < nbr ? rp[row] : 0, len = row < nbr ? rp[row + 1] - beg : 0;
+      const int pad = len > 0 ? cols[beg] : min (row, nbr - 1);
+      const int o = off[s], w = off[s + 1] - o;
+      for (int k = 0; k < w; k++)
+        {
+          const size_t at = ((size_t) (o + k) * kSlice + lane) * 2;
+          const bool in = k < len;
+          svals[at] = in ? vals[(size_t) (beg + k) * 4 + (lane & 1) * 2] : (T) 0;
+          svals[at + 1] = in ? vals[(size_t) (beg + k) * 4 + (lane & 1) * 2 + 1] : (T) 0;
+          if ((lane & 1) == 0)
+            scols[(size_t) (o + k) * (kSlice / 2) + lane / 2] = in ? cols[beg + k] : pad;
+        }
+    }
+}
 
 template <typename T, int BSC, class XL = dev::XNc> struct TprOp
 {
@@ -262,16 +473,26 @@ template <typename T> struct EpiDot
 {
   const T *a;
   T acc = 0;
+  T ai = 0; // a[i], where the product routine asks for it ahead (pre)
+  __device__ void pre (int64_t i) { ai = a[i]; }
   __device__ void operator() (int64_t i, T y) { acc = fma (a[i], y, acc); }
+  __device__ void now (int64_t, T y) { acc = fma (ai, y, acc); }
 };
 
 template <typename T> struct EpiTS
 {
   const T *s;
   T ts = 0, tt = 0;
+  T si = 0;
+  __device__ void pre (int64_t i) { si = s[i]; }
   __device__ void operator() (int64_t i, T t)
   {
     ts = fma (s[i], t, ts);
+    tt = fma (t, t, tt);
+  }
+  __device__ void now (int64_t, T t)
+  {
+    ts = fma (si, t, ts);
     tt = fma (t, t, tt);
   }
 };
@@ -289,6 +510,8 @@ template <typename T> struct EpiResidual
     rr = fma ((double) ri, (double) ri, rr);
     bb = fma ((double) bi, (double) bi, bb);
   }
+  __device__ void pre (int64_t) {}
+  __device__ void now (int64_t i, T y) { (*this) (i, y); }
 };
 
 // Residual replacement: r = c - A g, with (rh, r) and (r, r).
@@ -305,24 +528,41 @@ template <typename T> struct EpiReplace
     rhr = fma (rh[i], ri, rhr);
     rr = fma (ri, ri, rr);
   }
+  __device__ void pre (int64_t) {}
+  __device__ void now (int64_t i, T y) { (*this) (i, y); }
 };
 
 // The scalars that open an iteration, from the sums of (rh, r), (r, r) and
 // nn: the convergence, limit and breakdown tests, the replacement decision
 // (nn = (g, g) after a replacement or at a run's start, which resets the
-// deviation bound; else (x', x')) and beta. One thread of the last CTA of
-// the kernel that completed the sums runs it. GB300's FP64 pipe is narrow
-// (about 1/58 of FP32): the divides and square roots run once per kernel,
-// not in every CTA.
-__device__ void decide (DevState *st, double rho, double rr, double nn, bool after_rep)
+// deviation bound; else (x', x')) and beta. The last CTA of the kernel that
+// completed the sums runs it, all threads. An FP64 divide or square root
+// takes about half a microsecond on GB300's narrow FP64 pipe, so the four of
+// them run side by side, one to a warp, and one thread decides.
+__device__ __forceinline__ void decide (DevState *st, double rho, double rr, double nn, bool after_rep,
+                                        double rho_prev)
 {
+  __shared__ double sh[4]; // rho / rho_prev, alpha / omega, ||r||, sqrt (nn)
+  static_assert (kWarps >= 4, "one warp per divide and square root");
+  const double eps = st->eps;
+  if (threadIdx.x == 0)
+    sh[0] = rho / rho_prev;
+  else if (threadIdx.x == 32)
+    sh[1] = st->alpha / st->omega;
+  else if (threadIdx.x == 64)
+    sh[2] = sqrt (rr);
+  else if (threadIdx.x == 96)
+    sh[3] = eps > 0.0 ? sqrt (nn) : 0.0;
+  __syncthreads ();
+  if (threadIdx.x != 0)
+    return;
+  const double nr = sh[2], root_nn = sh[3];
   if (st->norm_b < 0.0)
-    st->norm_b = sqrt (rr); // ||r0|| of a fresh solve
+    st->norm_b = nr; // ||r0|| of a fresh solve
   const double nb = st->norm_b;
   const double omega = st->omega;
   int status = kStateRunning;
   double beta = 0.0;
-  const double nr = sqrt (rr);
   if (nb == 0.0 || nr < st->tol * nb) // gpu/bicgstab.cu:512
     status = kStateConverged;
   else if (st->iter >= st->max_iter)
@@ -331,19 +571,18 @@ __device__ void decide (DevState *st, double rho, double rr, double nn, bool aft
     status = kStateBreakdown;
   else
     {
-      beta = rho / st->rho_prev * st->alpha / omega; // gpu/bicgstab.cu:451
+      beta = sh[0] * sh[1]; // gpu/bicgstab.cu:451
       if (!isfinite (beta))
         status = kStateBreakdown;
     }
   int rep = 0;
-  const double eps = st->eps;
   if (status == kStateRunning && eps > 0.0)
     {
       if (after_rep)
-        st->dev = st->dev0 = eps * (st->cA * sqrt (nn) + nr);
+        st->dev = st->dev0 = eps * (st->cA * root_nn + nr);
       else
         {
-          const double dev = st->dev + eps * (st->cA * sqrt (nn) + nr);
+          const double dev = st->dev + eps * (st->cA * root_nn + nr);
           rep = st->dev <= kReplaceThreshold * st->nr_prev && dev > kReplaceThreshold * nr && dev > 1.1 * st->dev0;
           st->dev = dev;
         }
@@ -453,15 +692,14 @@ __device__ __forceinline__ void tail_end (DevState *st, const double *part, int 
   double sv[3];
   const int ks[3] = { kRhR, kRR, rep ? kGG : kXX };
   sum_parts<3> (part, grid, ks, sv);
-  if (threadIdx.x == 0)
+  const double rho_prev = rep ? st->rho_prev : st->rho;
+  __syncthreads (); // rho_prev is read
+  if (threadIdx.x == 0 && !rep)
     {
-      if (!rep)
-        {
-          st->rho_prev = st->rho;
-          st->iter = st->iter + 1;
-        }
-      decide (st, sv[0], sv[1], sv[2], rep);
+      st->rho_prev = rho_prev;
+      st->iter = st->iter + 1;
     }
+  decide (st, sv[0], sv[1], sv[2], rep, rho_prev);
 }
 
 template <typename T, class Op>
@@ -564,8 +802,7 @@ __global__ void __launch_bounds__ (kThreads)
     return;
   double sv[3];
   sum_parts<3> (a.part, a.grid, ks, sv);
-  if (threadIdx.x == 0)
-    decide (st, sv[0], sv[1], sv[2], true);
+  decide (st, sv[0], sv[1], sv[2], true, 1.0);
 }
 
 // Preconditioner of the vector phases (right preconditioning, q = M^-1 p,
@@ -1102,7 +1339,8 @@ enum SpmvKind
   kFlat16,
   kFlat32,
   kTpr3,
-  kTprAny
+  kTprAny,
+  kSell2 // bs = 2 on the engine's sliced copy
 };
 
 template <typename T, int K, class XL = dev::XNc> struct OpOf;
@@ -1112,6 +1350,7 @@ template <typename T, class XL> struct OpOf<T, kCsr8, XL> { using type = CsrOp<T
 // shuffle-reduction adds (each FP64 warp instruction costs the same issue
 // time on GB300's narrow FP64 pipe however many lanes are active).
 template <typename T, class XL> struct OpOf<T, kFlat2, XL> { using type = FlatOp<T, 2, 2, XL>; };
+template <typename T, class XL> struct OpOf<T, kSell2, XL> { using type = SellOp<T, XL>; };
 template <typename T, class XL> struct OpOf<T, kFlat4, XL> { using type = FlatOp<T, 4, 4, XL>; };
 template <typename T, class XL> struct OpOf<T, kFlat8, XL> { using type = FlatOp<T, 8, 4, XL>; };
 template <typename T, class XL> struct OpOf<T, kFlat16, XL> { using type = FlatOp<T, 16, 8, XL>; };
@@ -1152,6 +1391,7 @@ void launch_spmv_dispatch (int kind, int phase, const Args<T> &a, cudaStream_t s
     {
     case kCsr8: launch_spmv_phase<T, kCsr8> (phase, a, s); break;
     case kFlat2: launch_spmv_phase<T, kFlat2> (phase, a, s); break;
+    case kSell2: launch_spmv_phase<T, kSell2> (phase, a, s); break;
     case kFlat4: launch_spmv_phase<T, kFlat4> (phase, a, s); break;
     case kFlat8: launch_spmv_phase<T, kFlat8> (phase, a, s); break;
     case kFlat16: launch_spmv_phase<T, kFlat16> (phase, a, s); break;
@@ -1168,7 +1408,7 @@ void launch_residual (int kind, const Args<T> &a, const T *x, const T *b, T *r, 
     {
 #define BMFP_RES(K) case K: residual_kernel<T, typename OpOf<T, K>::type><<<a.grid, kThreads, 0, s>>> (a, x, b, r, y); break;
       BMFP_RES (kCsr8) BMFP_RES (kFlat2) BMFP_RES (kFlat4) BMFP_RES (kFlat8) BMFP_RES (kFlat16)
-      BMFP_RES (kFlat32) BMFP_RES (kTpr3)
+      BMFP_RES (kFlat32) BMFP_RES (kTpr3) BMFP_RES (kSell2)
 #undef BMFP_RES
     default: residual_kernel<T, typename OpOf<T, kTprAny>::type><<<a.grid, kThreads, 0, s>>> (a, x, b, r, y); break;
     }
@@ -1201,6 +1441,9 @@ Args<T> make_args (const bmfp_matrix_s *A, int64_t n, void *x, void *r, void *rh
   a.part = part;
   a.grid = grid;
   a.st = st;
+  a.soff = a.scols = nullptr;
+  a.svals = nullptr;
+  a.nslices = 0;
   return a;
 }
 
@@ -1247,6 +1490,7 @@ template <typename T> const void *iterate_for (int kind, int pk)
     {
     case kCsr8: return iterate_for_pre<T, kCsr8> (pk);
     case kFlat2: return iterate_for_pre<T, kFlat2> (pk);
+    case kSell2: return iterate_for_pre<T, kSell2> (pk);
     case kFlat4: return iterate_for_pre<T, kFlat4> (pk);
     case kTpr3: return iterate_for_pre<T, kTpr3> (pk);
     case kTprAny: return iterate_for_pre<T, kTprAny> (pk);
@@ -1306,6 +1550,7 @@ WideEngine::~WideEngine ()
     cudaFree (ptr);
   cudaFree (part_);
   cudaFree (state_);
+  cudaFree (svals_);
   if (h_state_)
     cudaFreeHost (h_state_);
 }
@@ -1331,6 +1576,12 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   chunk_ = std::max (1, std::min (chunk, 256));
   n_ = (int64_t) A->n_rows * bs;
   spmv_kind_ = spmv_kind_for (A);
+  if (spmv_kind_ == kFlat2)
+    {
+      const int rc = build_sliced (stream);
+      if (rc != BMFP_SUCCESS)
+        return rc;
+    }
   // Flat phases need 16-byte aligned values; cudaMalloc'd handles always are.
   int dev = 0, sms = 0;
   BMFP_CUDA (cudaGetDevice (&dev));
@@ -1409,6 +1660,80 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   return iterate_ ? BMFP_SUCCESS : capture (capture_stream_);
 }
 
+// The sliced copy of a bs = 2 matrix: one more pass over it at creation and as
+// many bytes again, kept where rows of one slice differ so little that the
+// padding stays below an eighth (a structured grid's below 1 %) and it takes at
+// most a quarter of the free memory; the products walk the block rows
+// otherwise.
+int WideEngine::build_sliced (cudaStream_t s)
+{
+  const int nbr = A_->n_rows;
+  if (nbr == 0 || A_->nnz == 0)
+    return BMFP_SUCCESS;
+  const int ns = (nbr + kSlice / 2 - 1) / (kSlice / 2);
+  const size_t S = dtype_size (dtype_);
+  // Temporaries from the stream-ordered pool: a cudaFree here would wait for
+  // every other stream of the device (the server's lanes create solvers while
+  // others run).
+  unsigned long long *tmp = nullptr, total = 0;
+  BMFP_CUDA (cudaMallocAsync (&tmp, 8 + sizeof (int) * (2 * (size_t) ns + 1), s));
+  int *width = (int *) (tmp + 1), *off = width + ns;
+  sell_width_kernel<<<(ns + 255) / 256, 256, 0, s>>> (nbr, A_->d_row_ptr, ns, width);
+  sell_scan_kernel<<<1, 1024, 0, s>>> (ns, width, off, tmp);
+  cudaError_t e = cudaGetLastError ();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync (&total, tmp, 8, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess)
+    e = cudaStreamSynchronize (s);
+  const size_t blocks = (size_t) total * (kSlice / 2);
+  const size_t o_off = (4 * S + sizeof (int)) * blocks;
+  size_t mem_free = 0, mem_total = 0;
+  if (e == cudaSuccess)
+    e = cudaMemGetInfo (&mem_free, &mem_total);
+  if (e == cudaSuccess && o_off < mem_free / 4 && blocks <= (size_t) (A_->nnz + A_->nnz / 8 + 1024) && total <= INT32_MAX
+      && cudaMalloc (&svals_, o_off + sizeof (int) * ((size_t) ns + 1)) == cudaSuccess)
+    {
+      scols_ = (int *) ((char *) svals_ + 4 * S * blocks);
+      soff_ = (int *) ((char *) svals_ + o_off);
+      e = cudaMemcpyAsync (soff_, off, sizeof (int) * ((size_t) ns + 1), cudaMemcpyDeviceToDevice, s);
+      const int grid = std::min ((ns + 7) / 8, 152 * 8);
+      if (dtype_ == BMFP_R64F)
+        sell_fill_kernel<double><<<grid, 256, 0, s>>> (nbr, A_->d_row_ptr, A_->d_cols, (const double *) A_->d_vals, ns,
+                                                       off, scols_, (double *) svals_);
+      else
+        sell_fill_kernel<float><<<grid, 256, 0, s>>> (nbr, A_->d_row_ptr, A_->d_cols, (const float *) A_->d_vals, ns,
+                                                      off, scols_, (float *) svals_);
+      if (e == cudaSuccess)
+        e = cudaGetLastError ();
+    }
+  else
+    cudaGetLastError (); // no room: walk the block rows
+  cudaFreeAsync (tmp, s);
+  if (e != cudaSuccess)
+    return cuda_fail (e, "sliced copy of the matrix", __FILE__, __LINE__);
+  if (!svals_)
+    return BMFP_SUCCESS;
+  nslices_ = ns;
+  spmv_kind_ = kSell2;
+  return BMFP_SUCCESS;
+}
+
+// Every kernel argument, q and z being p and s where there is no
+// preconditioner.
+template <typename T> struct WideEngine::ArgsOf
+{
+  static Args<T> make (const WideEngine &e, void *q, void *z)
+  {
+    Args<T> a = make_args<T> (e.A_, e.n_, e.x_, e.r_, e.rh_, e.p_, e.v_, q, e.s_, z, e.t_, e.P_, e.g_, e.xp_, e.part_,
+                              e.grid_, e.state_);
+    a.soff = e.soff_;
+    a.scols = e.scols_;
+    a.svals = (const T *) e.svals_;
+    a.nslices = e.nslices_;
+    return a;
+  }
+};
+
 int WideEngine::launch_iterations (cudaStream_t s)
 {
   void *q = jacobi_ ? q_ : p_;
@@ -1428,14 +1753,14 @@ int WideEngine::launch_iterations (cudaStream_t s)
   if (dtype_ == BMFP_R64F)
     {
       Args<double> a
-        = make_args<double> (A_, n_, x_, r_, rh_, p_, v_, q, s_, z, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<double>::make (*this, q, z);
       void *args[] = { &a, &iters };
       e = cudaLaunchKernelExC (&cfg, iterate_, args);
     }
   else
     {
       Args<float> a
-        = make_args<float> (A_, n_, x_, r_, rh_, p_, v_, q, s_, z, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<float>::make (*this, q, z);
       void *args[] = { &a, &iters };
       e = cudaLaunchKernelExC (&cfg, iterate_, args);
     }
@@ -1451,7 +1776,7 @@ int WideEngine::launch_phase (int phase, cudaStream_t s)
   if (dtype_ == BMFP_R64F)
     {
       Args<double> a
-        = make_args<double> (A_, n_, x_, r_, rh_, p_, v_, q, s_, z, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<double>::make (*this, q, z);
       if (phase == 2 || phase == 4)
         launch_spmv_dispatch<double> (spmv_kind_, phase, a, s);
       else
@@ -1460,7 +1785,7 @@ int WideEngine::launch_phase (int phase, cudaStream_t s)
   else
     {
       Args<float> a
-        = make_args<float> (A_, n_, x_, r_, rh_, p_, v_, q, s_, z, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<float>::make (*this, q, z);
       if (phase == 2 || phase == 4)
         launch_spmv_dispatch<float> (spmv_kind_, phase, a, s);
       else
@@ -1505,7 +1830,7 @@ int WideEngine::start (bool zero, const void *c, double tol, int max_iter, doubl
   if (dtype_ == BMFP_R64F)
     {
       const Args<double> a
-        = make_args<double> (A_, n_, x_, r_, rh_, p_, v_, q, s_, z, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<double>::make (*this, q, z);
       if (zero)
         start_kernel<double, true><<<grid_, kThreads, 0, s>>> (a, (const double *) c, tol, max_iter, norm_b, iter0,
                                                                 eps, cA_, new_shadow ? 1 : 0);
@@ -1516,7 +1841,7 @@ int WideEngine::start (bool zero, const void *c, double tol, int max_iter, doubl
   else
     {
       const Args<float> a
-        = make_args<float> (A_, n_, x_, r_, rh_, p_, v_, q, s_, z, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<float>::make (*this, q, z);
       if (zero)
         start_kernel<float, true><<<grid_, kThreads, 0, s>>> (a, (const float *) c, tol, max_iter, norm_b, iter0,
                                                                eps, cA_, new_shadow ? 1 : 0);
@@ -1658,14 +1983,14 @@ int WideEngine::true_residual (const void *d_b, void *d_r, double *rr, double *b
   if (dtype_ == BMFP_R64F)
     {
       Args<double> a
-        = make_args<double> (A_, n_, x_, r_, rh_, p_, v_, p_, s_, s_, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<double>::make (*this, p_, s_);
       launch_residual<double> (spmv_kind_, a, (const double *) x_, (const double *) d_b, (double *) d_r,
                                (double *) t_, s);
     }
   else
     {
       Args<float> a
-        = make_args<float> (A_, n_, x_, r_, rh_, p_, v_, p_, s_, s_, t_, P_, g_, xp_, part_, grid_, state_);
+        = ArgsOf<float>::make (*this, p_, s_);
       launch_residual<float> (spmv_kind_, a, (const float *) x_, (const float *) d_b, (float *) d_r,
                               (float *) t_, s);
     }

@@ -143,7 +143,10 @@ public:
   const bmfp_matrix_s *matrix () const { return A_; }
 
 private:
+  template <typename T> struct ArgsOf;
+
   int capture (cudaStream_t stream);
+  int build_sliced (cudaStream_t stream);
   int launch_phase (int phase, cudaStream_t stream);
   int launch_iterations (cudaStream_t stream);
   int barrier_fault (cudaStream_t stream);
@@ -165,6 +168,9 @@ private:
   void *x_ = nullptr, *r_ = nullptr, *rh_ = nullptr, *p_ = nullptr, *v_ = nullptr;
   void *q_ = nullptr, *s_ = nullptr, *z_ = nullptr, *t_ = nullptr, *P_ = nullptr;
   void *g_ = nullptr, *xp_ = nullptr;
+  void *svals_ = nullptr; // sliced copy of a bs = 2 matrix (one allocation), or null
+  int *soff_ = nullptr, *scols_ = nullptr;
+  int nslices_ = 0;
   double *part_ = nullptr;
   size_t part_bytes_ = 0;
   DevState *state_ = nullptr;

@@ -109,6 +109,34 @@ def test_fp64_diag_dominant_any_block_size(lib, cuda, bs):
     assert np.linalg.norm(x - xd) / np.linalg.norm(xd) < 1e-9
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("spread", [0, 1, 12])
+@pytest.mark.parametrize("nbr", [1, 15, 16, 17, 301, 5000])
+def test_sliced_copy_of_block_size_two(lib, cuda, nbr, spread, precision):
+    """Rows of one slice equal, differing by a block (the engine multiplies by
+    its padded slices) and differing too much for that (it walks the block
+    rows), with the last slice full, short by a row and holding one."""
+    rng = np.random.default_rng(nbr + spread)
+    rows = []
+    for i in range(nbr):
+        k = min(nbr, 9 + int(rng.integers(0, spread + 1)))
+        rows.append(np.unique(np.concatenate([[i], (i + np.arange(k)) % nbr])))
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    c = np.concatenate(rows).astype(np.int32)
+    v = rng.uniform(-1, 1, (c.size, 2, 2))
+    own = np.repeat(np.arange(nbr), np.diff(rp)) == c
+    v[own] += 45.0 * np.eye(2)
+    v = v.reshape(-1)
+    dt = np.float64 if precision == "fp64" else np.float32
+    A = bm.Matrix.from_bcsr(rp, c, v.astype(dt), 2)
+    b = rng.uniform(-1, 1, 2 * nbr).astype(dt)
+    x, info = bm.Solver(A, precision, tol=1e-10 if precision == "fp64" else 1e-5).solve_host(b)
+    assert info["status"] == bm.SUCCESS, info
+    K = bcsr_dense_csr(rp, c, v, 2)
+    assert np.linalg.norm(b - K @ x) / np.linalg.norm(b) < (2e-10 if precision == "fp64" else 2e-5)
+    A.close()
+
+
 def test_csr_matrix_solve_like_the_reference(lib, orc, cuda):
     """The reference solves CSR (csr_matrix_class); bs = 0 handles go through
     the CSR phase kernels."""
