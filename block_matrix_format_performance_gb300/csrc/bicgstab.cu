@@ -28,9 +28,11 @@
 // a CUDA graph of five kernels per iteration (`chunk` iterations per graph),
 // or one persistent cooperative kernel per `chunk` iterations whose phases
 // are separated by grid barriers, the last CTA to reach a barrier doing the
-// phase's scalar work (the auto choice from kPersistentRows rows). The host
-// only polls the done flag between launches; phases after convergence return
-// at once.
+// phase's scalar work (the auto choice from kPersistentRows rows). Below that
+// the auto mode runs the same recurrences in one cooperative kernel whose CTAs
+// keep their rows' vectors in shared memory (resident.cuh). The host only
+// polls the done flag between launches; phases after convergence return at
+// once.
 //
 // Residual replacement with group update (van der Vorst and Ye 2000, see
 // DevState): the decision at the end of phase 5 tracks the deviation bound
@@ -52,8 +54,10 @@
 #include <cuda/atomic>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace bmfp
@@ -91,7 +95,7 @@ template <typename T> struct Args
   double *part;
   int grid;
   DevState *st;
-  // Sliced copy of a bs = 2 matrix (SellOp), or null.
+  // Sliced copy of a CSR or bs = 2 matrix (SellOp), or null.
   const int *soff, *scols;
   const T *svals;
   int nslices;
@@ -100,33 +104,70 @@ template <typename T> struct Args
 // Sum over a warp, the same on every lane: each value's mantissa shifted to
 // the largest exponent of the warp (five guard bits: more than the FP64 adds
 // of a butterfly keep), the integers added exactly in three limbs by redux,
-// one rounding at the end. A butterfly's five dependent warp-wide FP64 adds
-// take about 500 cycles and keep GB300's narrow FP64 pipe busy throughout;
-// this takes about 150 on the integer pipes. Zeros, subnormals, infinities and
-// NaN go to the butterfly.
-__device__ __forceinline__ double warp_sum (double v)
+// one rounding (to nearest, halves away from zero) where the result is put
+// together. A butterfly's five dependent warp-wide FP64 adds take 600 cycles
+// on GB300, whose FP64 pipe starts one warp's instruction per 64 cycles and SM
+// quarter, and keep that pipe busy throughout; this runs on the integer pipes.
+// Zeros, subnormals, infinities and NaN go to the butterfly.
+// NK values at a time: their chains of redux run side by side.
+template <int NK> __device__ __forceinline__ void warp_sums (const double (&v)[NK], double (&out)[NK])
 {
   constexpr unsigned kAll = 0xffffffffu;
-  const long long bits = __double_as_longlong (v);
-  const int ex = (int) ((bits >> 52) & 0x7ff);
-  const int top = (int) __reduce_max_sync (kAll, (unsigned) ex);
-  if (top < 64 || top > 2047 - 64)
-    {
+  int top[NK];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-        v += __shfl_xor_sync (kAll, v, off);
-      return v;
+  for (int k = 0; k < NK; k++)
+    top[k] = (int) __reduce_max_sync (kAll, (unsigned) ((__double2hiint (v[k]) >> 20) & 0x7ff));
+#pragma unroll
+  for (int k = 0; k < NK; k++)
+    {
+      const long long bits = __double_as_longlong (v[k]);
+      const int ex = (int) ((bits >> 52) & 0x7ff);
+      const int d = top[k] - ex;
+      long long m = ex ? ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 5 : 0;
+      m = d < 58 ? (m + ((1ll << d) >> 1)) >> d : 0;
+      if (bits < 0)
+        m = -m;
+      const unsigned lo = __reduce_add_sync (kAll, (unsigned) (m & 0xfffff));
+      const unsigned mid = __reduce_add_sync (kAll, (unsigned) ((m >> 20) & 0xfffff));
+      const int hi = __reduce_add_sync (kAll, (int) (m >> 40));
+      const long long sum = ((long long) hi << 40) + ((long long) mid << 20) + lo;
+      unsigned long long u = (unsigned long long) (sum < 0 ? -sum : sum);
+      const int lz = __clzll ((long long) u);
+      u <<= lz & 63;
+      const unsigned long long man = (u >> 11) + ((u >> 10) & 1); // 2^52 .. 2^53
+      const unsigned long long r = ((unsigned long long) (top[k] + 5 - lz) << 52) + man;
+      out[k] = __longlong_as_double (sum ? (long long) (r | (sum < 0 ? 1ull << 63 : 0)) : 0);
     }
-  const int d = top - ex;
-  long long m = ex ? ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 5 : 0;
-  m = d < 58 ? (m + ((1ll << d) >> 1)) >> d : 0;
-  if (bits < 0)
-    m = -m;
-  const unsigned lo = __reduce_add_sync (kAll, (unsigned) (m & 0xfffff));
-  const unsigned mid = __reduce_add_sync (kAll, (unsigned) ((m >> 20) & 0xfffff));
-  const int hi = __reduce_add_sync (kAll, (int) (m >> 40));
-  const long long sum = ((long long) hi << 40) + ((long long) mid << 20) + lo;
-  return (double) sum * __longlong_as_double ((long long) (top - 57) << 52);
+#pragma unroll
+  for (int k = 0; k < NK; k++)
+    if (top[k] < 64 || top[k] > 2047 - 64)
+      {
+        double a = v[k];
+        if (__any_sync (kAll, (__double_as_longlong (a) << 1) != 0))
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1)
+            a += __shfl_xor_sync (kAll, a, off);
+        out[k] = a;
+      }
+}
+
+__device__ __forceinline__ double warp_sum (double v)
+{
+  const double in[1] = { v };
+  double out[1];
+  warp_sums<1> (in, out);
+  return out[0];
+}
+
+// Tests of doubles on the integer pipes (a DSETP costs what a DFMA does).
+__device__ __forceinline__ bool is_zero (double v) { return (__double_as_longlong (v) << 1) == 0; }
+__device__ __forceinline__ bool is_finite (double v) { return ((__double2hiint (v) >> 20) & 0x7ff) != 0x7ff; }
+// a < b for a and b non-negative, infinite or NaN (false then).
+__device__ __forceinline__ bool less_abs (double a, double b)
+{
+  const unsigned long long ua = (unsigned long long) __double_as_longlong (a),
+                           ub = (unsigned long long) __double_as_longlong (b);
+  return ua < ub && ub <= 0x7ff0000000000000ull;
 }
 
 // done and rep_now in one load. Both are written by earlier kernels (done
@@ -160,13 +201,12 @@ __device__ __forceinline__ void sum_parts (const double *part, int grid, const i
 #pragma unroll
     for (int k = 0; k < NK; k++)
       acc[k] += __ldcg (part + ks[k] * grid + i);
+  double ws[NK];
+  warp_sums<NK> (acc, ws);
+  if (lane == 0)
 #pragma unroll
-  for (int k = 0; k < NK; k++)
-    {
-      const double s = warp_sum (acc[k]);
-      if (lane == 0)
-        sh_w[k][w] = s;
-    }
+    for (int k = 0; k < NK; k++)
+      sh_w[k][w] = ws[k];
   __syncthreads ();
   if (w < NK)
     {
@@ -210,13 +250,12 @@ __device__ __forceinline__ void store_parts (double (&v)[NK], double *part, int 
 {
   __shared__ double sh[NK][kWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double ws[NK];
+  warp_sums<NK> (v, ws);
+  if (lane == 0)
 #pragma unroll
-  for (int k = 0; k < NK; k++)
-    {
-      const double a = warp_sum (v[k]);
-      if (lane == 0)
-        sh[k][w] = a;
-    }
+    for (int k = 0; k < NK; k++)
+      sh[k][w] = ws[k];
   __syncthreads ();
 #pragma unroll
   for (int k = 0; k < NK; k++)
@@ -249,9 +288,9 @@ template <typename T, int BS, int G, class XL = dev::XNc> struct FlatOp
 // Scalar rows per slice of the sliced matrix: one warp, one row per lane.
 constexpr int kSlice = 32;
 
-// bs = 2 on the sliced copy: step k of a slice holds line r of the k-th block
-// of each of its 32 scalar rows side by side, so a warp reads 512 (FP32: 256)
-// consecutive bytes per step where the row-by-row walk of the block rows
+// Block size B = 1 (CSR) or 2 on the sliced copy: step k of a slice holds line r
+// of the k-th block of each of its 32 scalar rows side by side, so a warp reads
+// 512 (FP64, B = 2) consecutive bytes per step where the row-by-row walk of the block rows
 // touched 16 lines, and every lane runs the same number of steps. Three
 // steps' x in flight and the next three steps' values and columns behind
 // them: the walk is bound by latency otherwise. Rows are padded to the
@@ -259,31 +298,47 @@ constexpr int kSlice = 32;
 // 2000x500 Q4 grid, FP64, phases 2 and 4 by block rows and by slices: 84.5 and
 // 88.4 us -> 72.8 and 81.1 us (FP64 pipe 74 % -> 82 % busy, its work alone 61
 // and 64 us).
-template <typename T, class XL = dev::XNc> struct SellOp
+template <typename T, int B, class XL = dev::XNc> struct SellOp
 {
-  static constexpr int U = 3;
+  static constexpr int U = sizeof (T) == 4 ? 9 : B == 1 ? 6 : 3;
   struct Step
   {
-    T v0, v1;
+    T v[B];
     int c;
   };
   __device__ static __forceinline__ Step load (const T *v, const int *c, int k)
   {
     Step s;
-    if constexpr (sizeof (T) == 8)
+    if constexpr (B == 1)
+      s.v[0] = __ldcs (v + (size_t) k * kSlice);
+    else if constexpr (sizeof (T) == 8)
       {
         const double2 t = __ldcs (reinterpret_cast<const double2 *> (v) + (size_t) k * kSlice);
-        s.v0 = t.x;
-        s.v1 = t.y;
+        s.v[0] = t.x;
+        s.v[1] = t.y;
       }
     else
       {
-        const float2 t = __ldcs (reinterpret_cast<const float2 *> (v) + (size_t) k * kSlice);
-        s.v0 = t.x;
-        s.v1 = t.y;
+        const float2 t = __ldg (reinterpret_cast<const float2 *> (v) + (size_t) k * kSlice);
+        s.v[0] = t.x;
+        s.v[1] = t.y;
       }
-    s.c = __ldg (c + (size_t) k * (kSlice / 2));
+    s.c = __ldg (c + (size_t) k * (kSlice / B));
     return s;
+  }
+  __device__ static __forceinline__ void gather (const T *x, int c, T (&xv)[B])
+  {
+    if constexpr (B == 1)
+      xv[0] = XL::ld (x + c);
+    else
+      XL::ld2 (x + (size_t) c * 2, xv[0], xv[1]);
+  }
+  __device__ static __forceinline__ T add (const Step &s, const T (&xv)[B], T acc)
+  {
+#pragma unroll
+    for (int j = 0; j < B; j++)
+      acc = fma (s.v[j], xv[j], acc);
+    return acc;
   }
   template <class Epi>
   __device__ static void run (const Args<T> &a, const T *x, T *y, Epi &e)
@@ -306,8 +361,8 @@ template <typename T, class XL = dev::XNc> struct SellOp
         const int64_t i = (int64_t) slice * kSlice + lane;
         if (i < a.n)
           e.pre (i);
-        const T *v = a.svals + ((size_t) beg * kSlice + lane) * 2;
-        const int *c = a.scols + (size_t) beg * (kSlice / 2) + lane / 2;
+        const T *v = a.svals + ((size_t) beg * kSlice + lane) * B;
+        const int *c = a.scols + (size_t) beg * (kSlice / B) + lane / B;
         const int n = end - beg;
         T acc = 0;
         int k = 0;
@@ -320,42 +375,35 @@ template <typename T, class XL = dev::XNc> struct SellOp
             for (; k + 2 * U <= n; k += U)
               {
                 Step t[U];
-                T x0[U], x1[U];
+                T xv[U][B];
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                  XL::ld2 (x + (size_t) s[u].c * 2, x0[u], x1[u]);
+                  gather (x, s[u].c, xv[u]);
 #pragma unroll
                 for (int u = 0; u < U; u++)
                   t[u] = load (v, c, k + U + u);
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                  {
-                    acc = fma (s[u].v0, x0[u], acc);
-                    acc = fma (s[u].v1, x1[u], acc);
-                  }
+                  acc = add (s[u], xv[u], acc);
 #pragma unroll
                 for (int u = 0; u < U; u++)
                   s[u] = t[u];
               }
-            T x0[U], x1[U];
+            T xv[U][B];
 #pragma unroll
             for (int u = 0; u < U; u++)
-              XL::ld2 (x + (size_t) s[u].c * 2, x0[u], x1[u]);
+              gather (x, s[u].c, xv[u]);
 #pragma unroll
             for (int u = 0; u < U; u++)
-              {
-                acc = fma (s[u].v0, x0[u], acc);
-                acc = fma (s[u].v1, x1[u], acc);
-              }
+              acc = add (s[u], xv[u], acc);
             k += U;
           }
         for (; k < n; k++)
           {
             const Step s = load (v, c, k);
-            T x0, x1;
-            XL::ld2 (x + (size_t) s.c * 2, x0, x1);
-            acc = fma (s.v0, x0, acc);
-            acc = fma (s.v1, x1, acc);
+            T xv[B];
+            gather (x, s.c, xv);
+            acc = add (s, xv, acc);
           }
         if (i < a.n)
           {
@@ -373,14 +421,14 @@ template <typename T, class XL = dev::XNc> struct SellOp
 
 // The sliced copy's layout: slice widths (its longest row, in blocks), their
 // running sum by one CTA (off[nslices] the total), and the fill.
-__global__ void sell_width_kernel (int nbr, const int *rp, int nslices, int *width)
+__global__ void sell_width_kernel (int nbr, int per, const int *rp, int nslices, int *width)
 {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslices)
     return;
-  const int r1 = min (nbr, (s + 1) * (kSlice / 2));
+  const int r1 = min (nbr, (s + 1) * per);
   int w = 0;
-  for (int r = s * (kSlice / 2); r < r1; r++)
+  for (int r = s * per; r < r1; r++)
     w = max (w, rp[r + 1] - rp[r]);
   width[s] = w;
 }
@@ -416,7 +464,7 @@ __global__ void __launch_bounds__ (1024) sell_scan_kernel (int nslices, const in
     }
 }
 
-template <typename T>
+template <typename T, int B>
 __global__ void sell_fill_kernel (int nbr, const int *rp, const int *cols, const T *vals, int nslices, const int *off,
                                   int *scols, T *svals)
 {
@@ -424,18 +472,18 @@ __global__ void sell_fill_kernel (int nbr, const int *rp, const int *cols, const
   const int nw = (int) (gridDim.x * blockDim.x / 32);
   for (int s = (int) ((blockIdx.x * blockDim.x + threadIdx.x) / 32); s < nslices; s += nw)
     {
-      const int row = s * (kSlice / 2) + lane / 2;
+      const int row = s * (kSlice / B) + lane / B;
       const int beg = row < nbr ? rp[row] : 0, len = row < nbr ? rp[row + 1] - beg : 0;
       const int pad = len > 0 ? cols[beg] : min (row, nbr - 1);
       const int o = off[s], w = off[s + 1] - o;
       for (int k = 0; k < w; k++)
         {
-          const size_t at = ((size_t) (o + k) * kSlice + lane) * 2;
+          const size_t at = ((size_t) (o + k) * kSlice + lane) * B;
           const bool in = k < len;
-          svals[at] = in ? vals[(size_t) (beg + k) * 4 + (lane & 1) * 2] : (T) 0;
-          svals[at + 1] = in ? vals[(size_t) (beg + k) * 4 + (lane & 1) * 2 + 1] : (T) 0;
-          if ((lane & 1) == 0)
-            scols[(size_t) (o + k) * (kSlice / 2) + lane / 2] = in ? cols[beg + k] : pad;
+          for (int j = 0; j < B; j++)
+            svals[at + j] = in ? vals[(size_t) (beg + k) * B * B + (lane % B) * B + j] : (T) 0;
+          if (lane % B == 0)
+            scols[(size_t) (o + k) * (kSlice / B) + lane / B] = in ? cols[beg + k] : pad;
         }
     }
 }
@@ -532,61 +580,48 @@ template <typename T> struct EpiReplace
   __device__ void now (int64_t i, T y) { (*this) (i, y); }
 };
 
-// The scalars that open an iteration, from the sums of (rh, r), (r, r) and
-// nn: the convergence, limit and breakdown tests, the replacement decision
-// (nn = (g, g) after a replacement or at a run's start, which resets the
-// deviation bound; else (x', x')) and beta. The last CTA of the kernel that
-// completed the sums runs it, all threads. An FP64 divide or square root
-// takes about half a microsecond on GB300's narrow FP64 pipe, so the four of
-// them run side by side, one to a warp, and one thread decides.
-__device__ __forceinline__ void decide (DevState *st, double rho, double rr, double nn, bool after_rep,
-                                        double rho_prev)
+// The scalars that open an iteration, from the sums of (rh, r), (r, r) and nn
+// ((g, g) after a replacement or at a run's start, which resets the deviation
+// bound; else (x', x')): the convergence, limit and breakdown tests, the
+// replacement decision and beta. One thread runs it, given the divides and
+// square roots: rho / rho_prev, alpha / omega, ||r|| and sqrt (nn).
+__device__ __forceinline__ void decide_scalars (DevState *st, double rho, double rr, double rho_ratio, double step_ratio,
+                                                double nr, double root_nn, bool after_rep)
 {
-  __shared__ double sh[4]; // rho / rho_prev, alpha / omega, ||r||, sqrt (nn)
-  static_assert (kWarps >= 4, "one warp per divide and square root");
   const double eps = st->eps;
-  if (threadIdx.x == 0)
-    sh[0] = rho / rho_prev;
-  else if (threadIdx.x == 32)
-    sh[1] = st->alpha / st->omega;
-  else if (threadIdx.x == 64)
-    sh[2] = sqrt (rr);
-  else if (threadIdx.x == 96)
-    sh[3] = eps > 0.0 ? sqrt (nn) : 0.0;
-  __syncthreads ();
-  if (threadIdx.x != 0)
-    return;
-  const double nr = sh[2], root_nn = sh[3];
-  if (st->norm_b < 0.0)
-    st->norm_b = nr; // ||r0|| of a fresh solve
-  const double nb = st->norm_b;
-  const double omega = st->omega;
+  double nb = st->norm_b;
+  if (nb < 0.0)
+    st->norm_b = nb = nr; // ||r0|| of a fresh solve
   int status = kStateRunning;
   double beta = 0.0;
-  if (nb == 0.0 || nr < st->tol * nb) // gpu/bicgstab.cu:512
+  if (is_zero (nb) || less_abs (nr, st->tol * nb)) // gpu/bicgstab.cu:512
     status = kStateConverged;
   else if (st->iter >= st->max_iter)
     status = kStateMaxIter;
-  else if (rho == 0.0 || omega == 0.0 || !isfinite (rho))
+  else if (is_zero (rho) || is_zero (st->omega) || !is_finite (rho))
     status = kStateBreakdown;
   else
     {
-      beta = sh[0] * sh[1]; // gpu/bicgstab.cu:451
-      if (!isfinite (beta))
+      beta = rho_ratio * step_ratio; // gpu/bicgstab.cu:451
+      if (!is_finite (beta))
         status = kStateBreakdown;
     }
   int rep = 0;
   if (status == kStateRunning && eps > 0.0)
     {
+      const double limit = kReplaceThreshold * nr;
       if (after_rep)
-        st->dev = st->dev0 = eps * (st->cA * root_nn + nr);
+        {
+          st->dev = eps * (st->cA * root_nn + nr);
+          st->dev_min = 1.1 * st->dev;
+        }
       else
         {
-          const double dev = st->dev + eps * (st->cA * root_nn + nr);
-          rep = st->dev <= kReplaceThreshold * st->nr_prev && dev > kReplaceThreshold * nr && dev > 1.1 * st->dev0;
+          const double dev = fma (eps, st->cA * root_nn + nr, st->dev);
+          rep = !less_abs (st->limit_prev, st->dev) && less_abs (limit, dev) && less_abs (st->dev_min, dev);
           st->dev = dev;
         }
-      st->nr_prev = nr;
+      st->limit_prev = limit;
     }
   st->rr = rr;
   if (status != kStateRunning)
@@ -605,6 +640,27 @@ __device__ __forceinline__ void decide (DevState *st, double rho, double rr, dou
       st->rho = rho;
       st->beta = beta;
     }
+}
+
+// The last CTA of the kernel that completed the sums runs this, all threads. An
+// FP64 divide or square root takes about 700 cycles on GB300's narrow FP64
+// pipe, so the four of them run side by side, one to a warp.
+__device__ __forceinline__ void decide (DevState *st, double rho, double rr, double nn, bool after_rep,
+                                        double rho_prev)
+{
+  __shared__ double sh[4];
+  static_assert (kWarps >= 4, "one warp per divide and square root");
+  if (threadIdx.x == 0)
+    sh[0] = rho / rho_prev;
+  else if (threadIdx.x == 32)
+    sh[1] = st->alpha / st->omega;
+  else if (threadIdx.x == 64)
+    sh[2] = sqrt (rr);
+  else if (threadIdx.x == 96)
+    sh[3] = st->eps > 0.0 ? sqrt (nn) : 0.0;
+  __syncthreads ();
+  if (threadIdx.x == 0)
+    decide_scalars (st, rho, rr, sh[0], sh[1], sh[2], sh[3], after_rep);
 }
 
 // Each phase is a body, run by every CTA, and (for phases that end in a dot
@@ -644,7 +700,7 @@ __device__ __forceinline__ void tail_v (DevState *st, const double *part, int gr
   if (threadIdx.x == 0)
     {
       const double alpha = st->rho / sv[0]; // gpu/bicgstab.cu:466
-      if (sv[0] != 0.0 && isfinite (alpha))
+      if (!is_zero (sv[0]) && is_finite (alpha))
         st->alpha = alpha;
       else
         {
@@ -672,8 +728,8 @@ __device__ __forceinline__ void tail_t (DevState *st, const double *part, int gr
   sum_parts<2> (part, grid, ks, sv);
   if (threadIdx.x == 0)
     {
-      const double omega = sv[1] != 0.0 ? sv[0] / sv[1] : 0.0; // :488
-      if (isfinite (omega))
+      const double omega = is_zero (sv[1]) ? 0.0 : sv[0] / sv[1]; // :488
+      if (is_finite (omega))
         st->omega = omega;
       else
         {
@@ -767,7 +823,7 @@ __global__ void __launch_bounds__ (kThreads)
       st->c = src;
       st->rep_now = 0;
       st->replacements = 0;
-      st->dev = st->dev0 = st->nr_prev = 0.0;
+      st->dev = st->dev_min = st->limit_prev = 0.0;
       if (ZERO)
         {
           st->iter = 0;
@@ -1165,6 +1221,8 @@ __global__ void __launch_bounds__ (kThreads, kIterateCtasPerSm) iterate_kernel (
     }
 }
 
+#include "resident.cuh"
+
 // The grid barrier's bounded wait, exercised: every CTA waits for one CTA
 // more than the grid holds, so no CTA is ever last; each gives up after
 // limit_ns, records the fault and returns, and the context stays usable.
@@ -1340,7 +1398,8 @@ enum SpmvKind
   kFlat32,
   kTpr3,
   kTprAny,
-  kSell2 // bs = 2 on the engine's sliced copy
+  kSell1, // CSR and bs = 2 on the engine's sliced copy
+  kSell2
 };
 
 template <typename T, int K, class XL = dev::XNc> struct OpOf;
@@ -1350,7 +1409,8 @@ template <typename T, class XL> struct OpOf<T, kCsr8, XL> { using type = CsrOp<T
 // shuffle-reduction adds (each FP64 warp instruction costs the same issue
 // time on GB300's narrow FP64 pipe however many lanes are active).
 template <typename T, class XL> struct OpOf<T, kFlat2, XL> { using type = FlatOp<T, 2, 2, XL>; };
-template <typename T, class XL> struct OpOf<T, kSell2, XL> { using type = SellOp<T, XL>; };
+template <typename T, class XL> struct OpOf<T, kSell1, XL> { using type = SellOp<T, 1, XL>; };
+template <typename T, class XL> struct OpOf<T, kSell2, XL> { using type = SellOp<T, 2, XL>; };
 template <typename T, class XL> struct OpOf<T, kFlat4, XL> { using type = FlatOp<T, 4, 4, XL>; };
 template <typename T, class XL> struct OpOf<T, kFlat8, XL> { using type = FlatOp<T, 8, 4, XL>; };
 template <typename T, class XL> struct OpOf<T, kFlat16, XL> { using type = FlatOp<T, 16, 8, XL>; };
@@ -1391,6 +1451,7 @@ void launch_spmv_dispatch (int kind, int phase, const Args<T> &a, cudaStream_t s
     {
     case kCsr8: launch_spmv_phase<T, kCsr8> (phase, a, s); break;
     case kFlat2: launch_spmv_phase<T, kFlat2> (phase, a, s); break;
+    case kSell1: launch_spmv_phase<T, kSell1> (phase, a, s); break;
     case kSell2: launch_spmv_phase<T, kSell2> (phase, a, s); break;
     case kFlat4: launch_spmv_phase<T, kFlat4> (phase, a, s); break;
     case kFlat8: launch_spmv_phase<T, kFlat8> (phase, a, s); break;
@@ -1408,7 +1469,7 @@ void launch_residual (int kind, const Args<T> &a, const T *x, const T *b, T *r, 
     {
 #define BMFP_RES(K) case K: residual_kernel<T, typename OpOf<T, K>::type><<<a.grid, kThreads, 0, s>>> (a, x, b, r, y); break;
       BMFP_RES (kCsr8) BMFP_RES (kFlat2) BMFP_RES (kFlat4) BMFP_RES (kFlat8) BMFP_RES (kFlat16)
-      BMFP_RES (kFlat32) BMFP_RES (kTpr3) BMFP_RES (kSell2)
+      BMFP_RES (kFlat32) BMFP_RES (kTpr3) BMFP_RES (kSell1) BMFP_RES (kSell2)
 #undef BMFP_RES
     default: residual_kernel<T, typename OpOf<T, kTprAny>::type><<<a.grid, kThreads, 0, s>>> (a, x, b, r, y); break;
     }
@@ -1490,12 +1551,26 @@ template <typename T> const void *iterate_for (int kind, int pk)
     {
     case kCsr8: return iterate_for_pre<T, kCsr8> (pk);
     case kFlat2: return iterate_for_pre<T, kFlat2> (pk);
+    case kSell1: return iterate_for_pre<T, kSell1> (pk);
     case kSell2: return iterate_for_pre<T, kSell2> (pk);
     case kFlat4: return iterate_for_pre<T, kFlat4> (pk);
     case kTpr3: return iterate_for_pre<T, kTpr3> (pk);
     case kTprAny: return iterate_for_pre<T, kTprAny> (pk);
     default: return nullptr;
     }
+}
+
+template <typename T, int B, int PK> const void *resident_for (bool matrix)
+{
+  return matrix ? reinterpret_cast<const void *> (&resident_kernel<T, B, PK, true>)
+                : reinterpret_cast<const void *> (&resident_kernel<T, B, PK, false>);
+}
+
+template <typename T> const void *resident_for (int kind, int pk, bool matrix)
+{
+  if (kind == kSell2)
+    return pk == kPrePoint ? resident_for<T, 2, kPrePoint> (matrix) : resident_for<T, 2, kPreNone> (matrix);
+  return pk == kPrePoint ? resident_for<T, 1, kPrePoint> (matrix) : resident_for<T, 1, kPreNone> (matrix);
 }
 
 // Unit roundoff of the engine's precision (replacement bound).
@@ -1551,12 +1626,14 @@ WideEngine::~WideEngine ()
   cudaFree (part_);
   cudaFree (state_);
   cudaFree (svals_);
+  cudaFree (resident_mem_);
+  cudaFree (resident_pub_);
   if (h_state_)
     cudaFreeHost (h_state_);
 }
 
 int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream_t stream, int ctas_per_sm,
-                      int launch_mode)
+                      int launch_mode, bool plain)
 {
   if (!A)
     return fail (BMFP_ERROR_INVALID_VALUE, "null matrix");
@@ -1571,12 +1648,13 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   dtype_ = A->dtype;
   jacobi_ = precond != BMFP_PRECOND_NONE;
   const bool block = precond == BMFP_PRECOND_BLOCK_JACOBI;
-  pre_kind_ = !jacobi_ ? kPreNone : !block ? kPrePoint : bs == 2 ? kPreBlock2 : kPreBlockAny;
+  // 1x1 blocks multiply elementwise (P holds the blocks' inverses).
+  pre_kind_ = !jacobi_ ? kPreNone : !block || bs == 1 ? kPrePoint : bs == 2 ? kPreBlock2 : kPreBlockAny;
   replace_ = dtype_ == BMFP_R64F;
   chunk_ = std::max (1, std::min (chunk, 256));
   n_ = (int64_t) A->n_rows * bs;
   spmv_kind_ = spmv_kind_for (A);
-  if (spmv_kind_ == kFlat2)
+  if (!plain && (spmv_kind_ == kFlat2 || spmv_kind_ == kCsr8))
     {
       const int rc = build_sliced (stream);
       if (rc != BMFP_SUCCESS)
@@ -1597,8 +1675,9 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   int cps = std::max (1, std::min (ctas_per_sm, 8));
   if (launch_mode == BMFP_LAUNCH_PERSISTENT || (launch_mode == BMFP_LAUNCH_AUTO && n_ >= kPersistentRows))
     {
-      const void *fn = dtype_ == BMFP_R64F ? iterate_for<double> (spmv_kind_, pre_kind_)
-                                           : iterate_for<float> (spmv_kind_, pre_kind_);
+      const void *fn = block                 ? nullptr
+                       : dtype_ == BMFP_R64F ? iterate_for<double> (spmv_kind_, pre_kind_)
+                                             : iterate_for<float> (spmv_kind_, pre_kind_);
       int coop = 0, per_sm = 0;
       BMFP_CUDA (cudaDeviceGetAttribute (&coop, cudaDevAttrCooperativeLaunch, dev));
       if (fn && coop)
@@ -1655,12 +1734,15 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   BMFP_CUDA (cudaEventCreateWithFlags (&ev_[1], cudaEventDisableTiming));
   BMFP_CUDA (cudaStreamCreateWithFlags (&capture_stream_, cudaStreamNonBlocking));
   int rc = matrix_bound (A, grid_, &cA_, stream); // synchronises the stream
+  if (rc == BMFP_SUCCESS && launch_mode == BMFP_LAUNCH_AUTO && !iterate_ && svals_ && n_ < kPersistentRows
+      && pre_kind_ <= kPrePoint)
+    rc = plan_resident (dev, sms, stream);
   if (rc != BMFP_SUCCESS)
     return rc;
   return iterate_ ? BMFP_SUCCESS : capture (capture_stream_);
 }
 
-// The sliced copy of a bs = 2 matrix: one more pass over it at creation and as
+// The sliced copy of a CSR or bs = 2 matrix: one more pass over it at creation and as
 // many bytes again, kept where rows of one slice differ so little that the
 // padding stays below an eighth (a structured grid's below 1 %) and it takes at
 // most a quarter of the free memory; the products walk the block rows
@@ -1670,7 +1752,8 @@ int WideEngine::build_sliced (cudaStream_t s)
   const int nbr = A_->n_rows;
   if (nbr == 0 || A_->nnz == 0)
     return BMFP_SUCCESS;
-  const int ns = (nbr + kSlice / 2 - 1) / (kSlice / 2);
+  const int B = spmv_kind_ == kFlat2 ? 2 : 1, per = kSlice / B;
+  const int ns = (nbr + per - 1) / per;
   const size_t S = dtype_size (dtype_);
   // Temporaries from the stream-ordered pool: a cudaFree here would wait for
   // every other stream of the device (the server's lanes create solvers while
@@ -1678,31 +1761,36 @@ int WideEngine::build_sliced (cudaStream_t s)
   unsigned long long *tmp = nullptr, total = 0;
   BMFP_CUDA (cudaMallocAsync (&tmp, 8 + sizeof (int) * (2 * (size_t) ns + 1), s));
   int *width = (int *) (tmp + 1), *off = width + ns;
-  sell_width_kernel<<<(ns + 255) / 256, 256, 0, s>>> (nbr, A_->d_row_ptr, ns, width);
+  sell_width_kernel<<<(ns + 255) / 256, 256, 0, s>>> (nbr, per, A_->d_row_ptr, ns, width);
   sell_scan_kernel<<<1, 1024, 0, s>>> (ns, width, off, tmp);
   cudaError_t e = cudaGetLastError ();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync (&total, tmp, 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
     e = cudaStreamSynchronize (s);
-  const size_t blocks = (size_t) total * (kSlice / 2);
-  const size_t o_off = (4 * S + sizeof (int)) * blocks;
+  const size_t blocks = (size_t) total * per;
+  const size_t o_off = (B * B * S + sizeof (int)) * blocks;
   size_t mem_free = 0, mem_total = 0;
   if (e == cudaSuccess)
     e = cudaMemGetInfo (&mem_free, &mem_total);
   if (e == cudaSuccess && o_off < mem_free / 4 && blocks <= (size_t) (A_->nnz + A_->nnz / 8 + 1024) && total <= INT32_MAX
       && cudaMalloc (&svals_, o_off + sizeof (int) * ((size_t) ns + 1)) == cudaSuccess)
     {
-      scols_ = (int *) ((char *) svals_ + 4 * S * blocks);
+      scols_ = (int *) ((char *) svals_ + B * B * S * blocks);
       soff_ = (int *) ((char *) svals_ + o_off);
       e = cudaMemcpyAsync (soff_, off, sizeof (int) * ((size_t) ns + 1), cudaMemcpyDeviceToDevice, s);
       const int grid = std::min ((ns + 7) / 8, 152 * 8);
+      auto fill = [&] (auto zero, auto width_c) {
+        using T = decltype (zero);
+        sell_fill_kernel<T, decltype (width_c)::value><<<grid, 256, 0, s>>> (
+          nbr, A_->d_row_ptr, A_->d_cols, (const T *) A_->d_vals, ns, off, scols_, (T *) svals_);
+      };
+      using One = std::integral_constant<int, 1>;
+      using Two = std::integral_constant<int, 2>;
       if (dtype_ == BMFP_R64F)
-        sell_fill_kernel<double><<<grid, 256, 0, s>>> (nbr, A_->d_row_ptr, A_->d_cols, (const double *) A_->d_vals, ns,
-                                                       off, scols_, (double *) svals_);
+        B == 2 ? fill (0.0, Two ()) : fill (0.0, One ());
       else
-        sell_fill_kernel<float><<<grid, 256, 0, s>>> (nbr, A_->d_row_ptr, A_->d_cols, (const float *) A_->d_vals, ns,
-                                                      off, scols_, (float *) svals_);
+        B == 2 ? fill (0.0f, Two ()) : fill (0.0f, One ());
       if (e == cudaSuccess)
         e = cudaGetLastError ();
     }
@@ -1714,7 +1802,69 @@ int WideEngine::build_sliced (cudaStream_t s)
   if (!svals_)
     return BMFP_SUCCESS;
   nslices_ = ns;
-  spmv_kind_ = kSell2;
+  spmv_kind_ = B == 2 ? kSell2 : kSell1;
+  return BMFP_SUCCESS;
+}
+
+// The resident iteration kernel's plan, for the auto launch mode: a sliced
+// matrix, no preconditioner or point Jacobi, fewer rows than the persistent
+// kernel's, and vectors that fit the SMs' shared memory beside each other.
+int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
+{
+  const int B = spmv_kind_ == kSell2 ? 2 : 1;
+  const int64_t S = (int64_t) dtype_size (dtype_);
+  int coop = 0, most = 0;
+  BMFP_CUDA (cudaDeviceGetAttribute (&coop, cudaDevAttrCooperativeLaunch, dev));
+  BMFP_CUDA (cudaDeviceGetAttribute (&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  most -= 2048; // the kernel's own
+  ResidentPlan P{};
+  // At least four warps of rows: one per FP64 pipe of an SM.
+  P.rows = (int) std::max<int64_t> (128, ((n_ + sms - 1) / sms + kSlice - 1) / kSlice * kSlice);
+  P.grid = (int) ((n_ + P.rows - 1) / P.rows);
+  const int64_t vectors = 7 * S * P.rows;
+  if (!coop || vectors > most)
+    return BMFP_SUCCESS;
+  const size_t o_flags = sizeof (unsigned long long) * 2 * kSlotKinds * 2 * (size_t) P.grid;
+  const size_t o_need = (o_flags + sizeof (unsigned) * (size_t) P.grid + 15) / 16 * 16;
+  BMFP_CUDA (cudaMalloc (&resident_mem_, o_need + sizeof (int2) * ((size_t) P.grid + 1)));
+  resident_zero_ = o_need;
+  BMFP_CUDA (cudaMemsetAsync (resident_mem_, 0, o_need + sizeof (int2) * ((size_t) P.grid + 1), s));
+  P.slots = (unsigned long long *) resident_mem_;
+  P.flags = (unsigned *) ((char *) resident_mem_ + o_flags);
+  int2 *need = (int2 *) ((char *) resident_mem_ + o_need), steps{};
+  P.need = need;
+  resident_need_kernel<<<P.grid, 256, 0, s>>> (n_, P.rows, B, soff_, scols_, need);
+  BMFP_LAUNCH_CHECK ();
+  BMFP_CUDA (cudaMemcpyAsync (&steps, need + P.grid, sizeof steps, cudaMemcpyDeviceToHost, s));
+  BMFP_CUDA (cudaStreamSynchronize (s));
+  const int64_t vals = (int64_t) steps.x * kSlice * B * S, cols = (int64_t) steps.x * (kSlice / B) * 4;
+  P.o_vals = (int) ((vectors + 15) / 16 * 16);
+  // Staged and with tagged words up to 640 rows a CTA (97 000 in all): there
+  // the waits count (us per FP64 iteration at 80 000 rows 27.8, 29.3 as
+  // graphs); above, the tags' traffic does (180 000 rows 41.5 against 37.8).
+  P.matrix = P.rows <= 640 && P.o_vals + vals + cols <= most;
+  P.threads = std::min (P.rows, resident_threads ((int) S, P.matrix));
+  P.o_cols = P.matrix ? (int) (P.o_vals + vals) : 0;
+  P.smem = (int) (P.matrix ? P.o_vals + vals + cols : vectors);
+  if (P.matrix)
+    {
+      // p and s as tagged words: a tag beside every four bytes
+      const size_t vec = (size_t) S * 2 * (size_t) n_;
+      resident_pub_bytes_ = 2 * vec;
+      BMFP_CUDA (cudaMalloc (&resident_pub_, resident_pub_bytes_));
+      BMFP_CUDA (cudaMemsetAsync (resident_pub_, 0, resident_pub_bytes_, s));
+      P.pub[0] = (unsigned long long *) resident_pub_;
+      P.pub[1] = (unsigned long long *) ((char *) resident_pub_ + vec);
+    }
+  const void *fn = dtype_ == BMFP_R64F ? resident_for<double> (spmv_kind_, pre_kind_, P.matrix)
+                                       : resident_for<float> (spmv_kind_, pre_kind_, P.matrix);
+  int per_sm = 0;
+  BMFP_CUDA (cudaFuncSetAttribute (fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  BMFP_CUDA (cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, fn, P.threads, (size_t) P.smem));
+  if ((int64_t) per_sm * sms < P.grid)
+    return BMFP_SUCCESS; // the graph then
+  resident_ = P;
+  iterate_ = fn;
   return BMFP_SUCCESS;
 }
 
@@ -1740,9 +1890,10 @@ int WideEngine::launch_iterations (cudaStream_t s)
   void *z = jacobi_ ? z_ : s_;
   int iters = chunk_;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3 ((unsigned) grid_);
-  cfg.blockDim = dim3 (kThreads);
-  cfg.dynamicSmemBytes = 0;
+  const bool res = resident_.grid > 0;
+  cfg.gridDim = dim3 ((unsigned) (res ? resident_.grid : grid_));
+  cfg.blockDim = dim3 ((unsigned) (res ? resident_.threads : kThreads));
+  cfg.dynamicSmemBytes = (size_t) resident_.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -1750,20 +1901,14 @@ int WideEngine::launch_iterations (cudaStream_t s)
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e;
+  auto launch = [&] (auto a) {
+    void *plain[] = { &a, &iters }, *planned[] = { &a, &resident_, &iters };
+    return cudaLaunchKernelExC (&cfg, iterate_, res ? planned : plain);
+  };
   if (dtype_ == BMFP_R64F)
-    {
-      Args<double> a
-        = ArgsOf<double>::make (*this, q, z);
-      void *args[] = { &a, &iters };
-      e = cudaLaunchKernelExC (&cfg, iterate_, args);
-    }
+    e = launch (ArgsOf<double>::make (*this, q, z));
   else
-    {
-      Args<float> a
-        = ArgsOf<float>::make (*this, q, z);
-      void *args[] = { &a, &iters };
-      e = cudaLaunchKernelExC (&cfg, iterate_, args);
-    }
+    e = launch (ArgsOf<float>::make (*this, q, z));
   if (e != cudaSuccess)
     return cuda_fail (e, "cooperative launch of the iteration kernel", __FILE__, __LINE__);
   return BMFP_SUCCESS;
@@ -1883,6 +2028,10 @@ int WideEngine::barrier_fault (cudaStream_t s)
   BMFP_CUDA (cudaStreamSynchronize (s));
   BMFP_CUDA (cudaMemsetAsync (state_, 0, sizeof (DevState), s));
   BMFP_CUDA (cudaMemsetAsync (part_, 0, part_bytes_, s));
+  if (resident_mem_)
+    BMFP_CUDA (cudaMemsetAsync (resident_mem_, 0, resident_zero_, s));
+  if (resident_pub_)
+    BMFP_CUDA (cudaMemsetAsync (resident_pub_, 0, resident_pub_bytes_, s));
   BMFP_CUDA (cudaStreamSynchronize (s));
   return fail (BMFP_ERROR_TIMEOUT, "a grid barrier of the iteration kernel gave up waiting");
 }

@@ -43,8 +43,8 @@ struct DevState
   double eps;      // unit roundoff of the working precision; 0 = no replacement
   double cA;       // max entries per scalar row * max absolute row sum
   double dev;      // deviation bound since the last replacement
-  double dev0;     // its value at the last replacement
-  double nr_prev;  // ||r|| at the previous decision
+  double dev_min;    // 1.1 times its value at the last replacement
+  double limit_prev; // kReplaceThreshold * ||r|| at the previous decision
   const void *c;   // right-hand side of the run (b, or a restart's residual)
   // done and rep_now side by side (8-byte aligned): every phase reads both
   // with one load at its start.
@@ -79,6 +79,23 @@ enum
   kStateBreakdown = 3
 };
 
+// Launch plan of the resident iteration kernel (resident.cuh).
+struct ResidentPlan
+{
+  int rows = 0; // scalar rows per CTA, a multiple of 32
+  int grid = 0, threads = 0;
+  bool matrix = false; // the CTA's part of the sliced matrix is staged in shared memory
+  int o_vals = 0, o_cols = 0; // byte offsets of that copy
+  int smem = 0;
+  unsigned long long *slots = nullptr; // words of the sums: [2][kSlotKinds][grid][2]
+  // With the matrix in shared memory, p (q, g) and s (z) are published as
+  // tagged words; else in place, a flag per CTA behind them, and a CTA waits
+  // for the flags of CTAs need.x to need.y, whose rows its columns belong to.
+  unsigned long long *pub[2] = {};
+  unsigned *flags = nullptr;
+  const int2 *need = nullptr; // [grid], then the most steps of any CTA's rows
+};
+
 // Whole-GPU BiCGStab on one matrix: five fused phases per iteration over all
 // rows on a fixed grid, either as phase kernels captured in a CUDA graph of
 // `chunk` iterations or as one persistent cooperative kernel per `chunk`
@@ -101,9 +118,11 @@ public:
   WideEngine &operator= (const WideEngine &) = delete;
 
   // precond: BMFP_PRECOND_NONE, _JACOBI (point) or _BLOCK_JACOBI (bs <= 8).
-  // launch_mode: enum bmfp_launch_mode.
+  // launch_mode: enum bmfp_launch_mode. plain: the matrix's own arrays and the
+  // phase kernels, as the allocation-free entry point runs them (no sliced
+  // copy, no resident kernel).
   int init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream_t stream, int ctas_per_sm = 4,
-            int launch_mode = 0);
+            int launch_mode = 0, bool plain = false);
   // Residual replacement on (default for FP64 engines) or off (the
   // reference's plain recurrences; FP32 engines always run without it).
   void set_replacement (bool on) { replace_ = on && dtype_ == BMFP_R64F; }
@@ -147,6 +166,7 @@ private:
 
   int capture (cudaStream_t stream);
   int build_sliced (cudaStream_t stream);
+  int plan_resident (int dev, int sms, cudaStream_t stream);
   int launch_phase (int phase, cudaStream_t stream);
   int launch_iterations (cudaStream_t stream);
   int barrier_fault (cudaStream_t stream);
@@ -176,7 +196,11 @@ private:
   DevState *state_ = nullptr;
   DevState *h_state_ = nullptr; // pinned, two slots
   cudaGraphExec_t graph_ = nullptr;
-  const void *iterate_ = nullptr; // persistent iteration kernel, or null: graphs
+  const void *iterate_ = nullptr; // persistent or resident iteration kernel, or null: graphs
+  ResidentPlan resident_;         // of the resident kernel (grid 0: not in use)
+  void *resident_mem_ = nullptr;  // its words, flags and ranges
+  void *resident_pub_ = nullptr;  // its published vectors
+  size_t resident_zero_ = 0, resident_pub_bytes_ = 0; // bytes a fault clears
   cudaStream_t capture_stream_ = nullptr;
   cudaEvent_t ev_[2] = { nullptr, nullptr };
 };

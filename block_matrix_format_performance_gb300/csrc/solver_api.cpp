@@ -401,6 +401,10 @@ int bmfp_solver_create (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_o
   sv->opts = o;
   sv->A = A;
   const int jac = o.preconditioner;
+  // Without the true-residual check (the reference's stopping rule) a solve
+  // takes the iterations of the allocation-free entry point, which has no
+  // room for a copy of the matrix: the same kernels on the same arrays.
+  const bool plain = o.check_true_residual == 0;
   int rc = BMFP_SUCCESS;
   const bmfp_matrix_s *A32 = A;
   if (o.precision != BMFP_SOLVE_FP64 && A->dtype == BMFP_R64F)
@@ -413,16 +417,16 @@ int bmfp_solver_create (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_o
   if (o.precision == BMFP_SOLVE_FP32)
     {
       sv->main.reset (new (std::nothrow) WideEngine);
-      rc = sv->main->init (A32, jac, o.iterations_per_graph, s, o.ctas_per_sm, o.launch_mode);
+      rc = sv->main->init (A32, jac, o.iterations_per_graph, s, o.ctas_per_sm, o.launch_mode, plain);
     }
   else
     {
       sv->main.reset (new (std::nothrow) WideEngine);
-      rc = sv->main->init (A, jac, o.iterations_per_graph, s, o.ctas_per_sm, o.launch_mode);
+      rc = sv->main->init (A, jac, o.iterations_per_graph, s, o.ctas_per_sm, o.launch_mode, plain);
       if (rc == BMFP_SUCCESS && o.precision == BMFP_SOLVE_MIXED)
         {
           sv->inner.reset (new (std::nothrow) WideEngine);
-          rc = sv->inner->init (A32, jac, o.iterations_per_graph, s, o.ctas_per_sm, o.launch_mode);
+          rc = sv->inner->init (A32, jac, o.iterations_per_graph, s, o.ctas_per_sm, o.launch_mode, plain);
         }
     }
   if (rc != BMFP_SUCCESS)

@@ -279,7 +279,11 @@ enum bmfp_preconditioner
 
 enum bmfp_launch_mode
 {
-  BMFP_LAUNCH_AUTO = 0,       /* persistent from 1 000 000 rows up when it can run, else graphs */
+  BMFP_LAUNCH_AUTO = 0,       /* persistent from 1 000 000 rows up when it can run; below, for CSR
+                                 and bs = 2 without block Jacobi, one cooperative kernel per
+                                 iterations_per_graph iterations that keeps the Krylov vectors in
+                                 shared memory, where they fit (about 600 000 rows in FP64) and
+                                 check_true_residual is 1; else graphs */
   BMFP_LAUNCH_GRAPH = 1,      /* a CUDA graph of five phase kernels per iteration */
   BMFP_LAUNCH_PERSISTENT = 2  /* one cooperative kernel per iterations_per_graph iterations, the
                                  phases separated by grid barriers, over min(ctas_per_sm, 3) CTAs
@@ -316,10 +320,11 @@ typedef struct bmfp_solver_options
                                b - A x; applies when check_true_residual is 1 (with 0 the
                                reference's plain recurrences run) */
   int launch_mode;          /* enum bmfp_launch_mode (default AUTO). On the same grid (ctas_per_sm
-                               <= 3) both modes give the same bits. The persistent kernel holds
-                               every SM for its launch, so other work on the GPU waits for it
-                               (the server's lanes, which share the GPU with the batched
-                               solver, use graphs) */
+                               <= 3) the graph and the persistent mode give the same bits; the
+                               auto mode's shared-memory kernel has a grid of its own. The
+                               cooperative kernels hold the SMs they run on for a launch, so
+                               other work waits for them (the server's lanes, which share the
+                               GPU with the batched solver, use graphs) */
 } bmfp_solver_options;
 
 typedef struct bmfp_solve_info

@@ -546,6 +546,84 @@ def test_auto_launch_mode_takes_the_persistent_kernel_from_a_million_rows(lib, c
     A.close()
 
 
+def shifted_q4(nx, ny, shift=0.02):
+    rp, c, v, _ = bm.gen_q4_elasticity(nx, ny)
+    rows = np.repeat(np.arange(nx * ny), np.diff(rp))
+    v.reshape(-1, 2, 2)[c == rows] += shift * np.eye(2)
+    return rp, c, v
+
+
+@pytest.mark.parametrize("fmt", ["bcsr", "csr"])
+@pytest.mark.parametrize("precision,precond", [("fp64", "none"), ("fp64", "jacobi"), ("mixed", "none")])
+@pytest.mark.parametrize("grid", [(2, 2), (9, 7), (16, 4), (13, 5), (150, 65), (201, 243), (251, 250), (700, 201)])
+def test_auto_mode_on_systems_that_fit_the_sms(lib, cuda, grid, precision, precond, fmt):
+    """The auto launch mode's kernel for systems whose vectors fit the SMs'
+    shared memory, from one partly filled CTA over the staged matrix's limit
+    (640 rows a CTA) to several thousand rows a CTA: the graph's answer, and
+    the same bits every time."""
+    import torch
+    rp, c, v = shifted_q4(*grid)
+    n = 2 * grid[0] * grid[1]
+    if fmt == "csr":
+        A = bm.Matrix.from_csr(*bm.bcsr_to_csr(rp, c, v, 2), n)
+    else:
+        A = bm.Matrix.from_bcsr(rp, c, v, 2)
+    b = dev(np.random.default_rng(n).uniform(-1, 1, n))
+    out = {}
+    for mode in ("auto", "graph"):
+        s = bm.Solver(A, precision, tol=1e-12, preconditioner=precond, launch_mode=mode)
+        x = torch.empty_like(b)
+        info = s.solve(b, x)
+        again = torch.empty_like(b)
+        s.solve(b, again)
+        assert info["status"] == bm.SUCCESS and info["true_rel_residual"] < 1e-12, (mode, info)
+        assert torch.equal(x.view(torch.int64), again.view(torch.int64)), mode
+        out[mode] = x, info
+        s.close()
+    (xa, ia), (xg, ig) = out["auto"], out["graph"]
+    # ||x - x'|| <= 2 tol ||b|| / sigma_min, sigma_min >= the shift
+    assert torch.linalg.norm(xa - xg) <= 2e-12 * torch.linalg.norm(b) / 0.02
+    assert abs(ia["iterations"] - ig["iterations"]) <= 0.25 * ig["iterations"] + 10
+    A.close()
+
+
+def test_auto_mode_solves_on_separate_streams(lib, cuda):
+    """Four auto solves at once from four threads on four streams, staged and
+    unstaged: each has the bits of the same solve run alone."""
+    import threading
+    import torch
+    work = []
+    for grid in ((40, 30), (150, 65), (251, 250), (400, 150)):
+        rp, c, v = shifted_q4(*grid)
+        A = bm.Matrix.from_bcsr(rp, c, v, 2)
+        b = dev(np.random.default_rng(grid[0]).uniform(-1, 1, 2 * grid[0] * grid[1]))
+        x = torch.empty_like(b)
+        bm.Solver(A, "fp64", tol=1e-12).solve(b, x)
+        work.append((A, b, x))
+    torch.cuda.synchronize()
+    out = {}
+
+    def worker(k):
+        A, b, _ = work[k]
+        st = torch.cuda.Stream()
+        s = bm.Solver(A, "fp64", tol=1e-12, stream=st.cuda_stream)
+        x = torch.empty_like(b)
+        for _ in range(5):
+            info = s.solve(b, x, stream=st.cuda_stream)
+        st.synchronize()
+        out[k] = info, x
+
+    threads = [threading.Thread(target=worker, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(4):
+        info, x = out[k]
+        assert info["status"] == bm.SUCCESS, info
+        assert torch.equal(x.view(torch.int64), work[k][2].view(torch.int64))
+
+
 def test_concurrent_persistent_solves_on_separate_streams(lib, cuda):
     """Three persistent solves of a 1 000 000-row system launched at once from
     three host threads on three streams: cooperative launches that cannot be
