@@ -25,6 +25,7 @@
 // shared through shared memory: GB300's FP64 pipe is too narrow to evaluate
 // divides and square roots in every thread.
 #include "batch.h"
+#include "reduce.cuh"
 #include "spmv_core.cuh"
 
 #include <cooperative_groups.h>
@@ -39,65 +40,52 @@ namespace cg = cooperative_groups;
 
 namespace bmfp
 {
+using namespace reduce;
+
 namespace
 {
 constexpr int kMaxThreads = 1024;
 constexpr int kLaunchThreads = 512; // the batch kernel's launch bounds
 
-__device__ __forceinline__ double warp_sum_d (double v)
-{
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-    v += __shfl_xor_sync (0xffffffffu, v, off);
-  return v;
-}
-
-// Team-wide sums of NK values, fixed order: warps, then CTAs by rank.
+// Team-wide sums of NK values, in shared memory until the next call for NK
+// values (registers are short where they are needed): warps, then CTAs, by exact integer sums (the
+// order does not matter). Each CTA writes its totals into every CTA's shared
+// memory, so one cluster barrier per call publishes them all; successive calls
+// take two sets of them in turn (`turn`): a CTA one call ahead cannot overwrite
+// what another still reads. Thread 0 adding sixteen warps' and then eight CTAs'
+// totals one by one took about 1500 cycles per value, each FP64 add 64 of them,
+// between two cluster barriers.
 template <int NK>
-__device__ void team_sum (cg::cluster_group &cl, double (&v)[NK], double (&out)[NK])
+__device__ const double *team_sum (cg::cluster_group &cl, int &turn, double (&v)[NK])
 {
-  __shared__ double sh_w[NK][kMaxThreads / 32];
-  __shared__ double sh_cta[NK];
+  __shared__ double sh_w[NK][32];
+  __shared__ double sh_cta[2][NK][8];
+  __shared__ double sh_sum[NK];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    {
-      const double s = warp_sum_d (v[k]);
-      if (lane == 0)
-        sh_w[k][w] = s;
-    }
-  __syncthreads ();
-  if (threadIdx.x == 0)
+  const int size = (int) cl.num_blocks (), rank = (int) cl.block_rank ();
+  double ws[NK];
+  warp_sums<NK> (v, ws);
+  if (lane == 0)
 #pragma unroll
     for (int k = 0; k < NK; k++)
-      {
-        double a = 0.0;
-        for (int i = 0; i < nw; i++)
-          a += sh_w[k][i];
-        sh_cta[k] = a;
-      }
-  cl.sync ();
-  // Thread 0 adds the CTAs' totals in rank order; the second cluster barrier
-  // publishes the sum to the CTA and keeps sh_cta alive until every CTA has
-  // read it. (Every thread summing the ranks itself issued size warp-wide
-  // FP64 adds per warp and value on GB300's narrow FP64 pipe.)
-  __shared__ double sh_sum[NK];
-  if (threadIdx.x == 0)
+      sh_w[k][w] = ws[k];
+  __syncthreads ();
+  for (int k = w; k < NK; k += nw)
     {
-      const unsigned size = cl.num_blocks ();
-#pragma unroll
-      for (int k = 0; k < NK; k++)
-        {
-          double a = 0.0;
-          for (unsigned r = 0; r < size; r++)
-            a += *cl.map_shared_rank (&sh_cta[k], r);
-          sh_sum[k] = a;
-        }
+      const double a = warp_sum (lane < nw ? sh_w[k][lane] : 0.0);
+      if (lane < size)
+        *cl.map_shared_rank (&sh_cta[turn][k][rank], lane) = a;
     }
   cl.sync ();
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    out[k] = sh_sum[k];
+  for (int k = w; k < NK; k += nw)
+    {
+      const double a = warp_sum (lane < size ? sh_cta[turn][k][lane] : 0.0);
+      if (lane == 0)
+        sh_sum[k] = a;
+    }
+  turn ^= 1;
+  __syncthreads ();
+  return sh_sum;
 }
 
 // Team-wide maxima of NK non-negative values.
@@ -178,8 +166,73 @@ template <typename T> struct TeamOp<T, kOpFlat2>
   template <class Epi>
   __device__ static void run (const TeamSys<T> &S, const TeamIdx &ix, const T *x, T *y, Epi &e)
   {
-    for (int64_t row = ix.group0; row < S.nbr; row += ix.group_stride)
-      core::flat_row<T, 2, 2, 4> ((int) row, S.rp, S.cols, S.vals, x, y, e);
+    if constexpr (sizeof (T) == 4)
+      pair_rows (S, ix, x, y, e);
+    else
+      for (int64_t row = ix.group0; row < S.nbr; row += ix.group_stride)
+        core::flat_row<T, 2, 2, 4> ((int) row, S.rp, S.cols, S.vals, x, y, e);
+  }
+  // FP32: two lanes share a block row, a whole block each per step, five steps
+  // (ten blocks: a row of a Q4 grid) at once, the next row's offsets ahead. A
+  // few rows per thread, so a row's round trips are what the product takes.
+  template <class Epi>
+  __device__ static __forceinline__ void pair_rows (const TeamSys<float> &S, const TeamIdx &ix, const float *x,
+                                                    float *y, Epi &e)
+  {
+    constexpr int U = 5;
+    const int gl = threadIdx.x & 1;
+    const unsigned mask = dev::group_mask<2> ();
+    int64_t row = ix.group0;
+    if (row >= S.nbr)
+      return;
+    int beg = __ldg (S.rp + row), end = __ldg (S.rp + row + 1);
+    for (;;)
+      {
+        const int64_t next = row + ix.group_stride;
+        int nbeg = 0, nend = 0;
+        if (next < S.nbr)
+          {
+            nbeg = __ldg (S.rp + next);
+            nend = __ldg (S.rp + next + 1);
+          }
+        float a0 = 0, a1 = 0;
+        for (int b0 = beg + gl; b0 < end; b0 += 2 * U)
+          {
+            // past the row's end: its last block again, not added
+            float4 av[U];
+            float2 xv[U];
+            int c[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+              {
+                const int b = min (b0 + 2 * u, end - 1);
+                c[u] = __ldg (S.cols + b);
+                av[u] = __ldcs (reinterpret_cast<const float4 *> (S.vals) + b);
+              }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+              xv[u] = __ldg (reinterpret_cast<const float2 *> (x) + c[u]);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+              if (b0 + 2 * u < end)
+                {
+                  a0 = fmaf (av[u].x, xv[u].x, a0);
+                  a0 = fmaf (av[u].y, xv[u].y, a0);
+                  a1 = fmaf (av[u].z, xv[u].x, a1);
+                  a1 = fmaf (av[u].w, xv[u].y, a1);
+                }
+          }
+        // lane gl keeps scalar row gl of the block row
+        const float mine = gl ? a1 : a0, other = gl ? a0 : a1;
+        const float sum = mine + __shfl_xor_sync (mask, other, 1);
+        y[row * 2 + gl] = sum;
+        e (row * 2 + gl, sum);
+        if (next >= S.nbr)
+          break;
+        row = next;
+        beg = nbeg;
+        end = nend;
+      }
   }
 };
 template <typename T> struct TeamOp<T, kOpCsr>
@@ -219,7 +272,7 @@ template <typename T> struct EpiDotT
 {
   const T *a;
   double acc = 0.0;
-  __device__ void operator() (int64_t i, T y) { acc = fma ((double) a[i], (double) y, acc); }
+  __device__ void operator() (int64_t i, T y) { acc = fma (widen (a[i]), widen (y), acc); }
 };
 template <typename T> struct EpiTST
 {
@@ -227,8 +280,9 @@ template <typename T> struct EpiTST
   double ts = 0.0, tt = 0.0;
   __device__ void operator() (int64_t i, T t)
   {
-    ts = fma ((double) s[i], (double) t, ts);
-    tt = fma ((double) t, (double) t, tt);
+    const double td = widen (t);
+    ts = fma (widen (s[i]), td, ts);
+    tt = fma (td, td, tt);
   }
 };
 struct EpiResid
@@ -294,12 +348,24 @@ struct SolveOut
   double rec_rel = 0.0;
 };
 
-// Thread 0 of each CTA evaluates the scalars; the rest read them here.
+// A run's scalars, in shared memory: the divides and square roots are taken by
+// four warps of each CTA side by side and the decisions by thread 0; every CTA
+// of the team computes the same from the same sums. (Kept per thread they took
+// some thirty of the kernel's 64 registers from the loads in flight.)
 struct Scal
 {
-  double a, b, c;
+  double rho, rho_prev, alpha, omega, rr, nn; // nn: (x', x'), or (g, g) after a replacement
+  double nb;                                  // reference norm
+  double rho_ratio, step_ratio, nr, root_nn;
+  double beta, rel;
+  // thread 0's: the best (r, r) and 1e16 of it, a quarter of the one at the last
+  // halving, that of the copy and a quarter of it, and the replacement bound
+  double best_rr, blow_rr, mark_4th, snap_rr, snap_4th, dev, dev_min, limit_prev;
+  int mark_it, reset;
   int status;
-  int rep; // replace r by the true residual before the next iteration
+  int rep;     // replace r by the true residual before the next iteration
+  int snap;    // copy the iterate
+  int restore; // the run ended above its copy
 };
 
 // One BiCGStab solve by the team. r0 = rhs (x updated in place from x0 = 0
@@ -327,12 +393,16 @@ struct Scal
 // by the true residual bt - A x (bt: the system's b). Applied at once, in the
 // iteration where the bound crosses.
 template <typename T, int OP, bool RR = false>
-__device__ SolveOut team_bicgstab (cg::cluster_group &cl, const TeamSys<T> &S, const T *rhs, T *x, bool zero_x,
+__device__ SolveOut team_bicgstab (cg::cluster_group &cl, int &turn, const TeamSys<T> &S, const T *rhs, T *x, bool zero_x,
                                    double tol, int max_it, double norm_ref, T *snap = nullptr, int stall = 0,
                                    const T *bt = nullptr, T *xp = nullptr, double cA = 0.0, int *reps = nullptr,
                                    bool new_shadow = false)
 {
   using Op = TeamOp<T, OP>;
+  // Rows of the vector updates a thread loads at once (the stores may alias
+  // the next rows' loads as far as the compiler knows); past the end its first
+  // row again, not stored.
+  constexpr int kRows = 4;
   const TeamIdx ix = team_index<Op::G> (cl);
   __shared__ Scal sc;
   SolveOut o;
@@ -353,87 +423,117 @@ __device__ SolveOut team_bicgstab (cg::cluster_group &cl, const TeamSys<T> &S, c
       rr0 = fma ((double) ri, (double) ri, rr0);
       rhr0 = fma ((double) hi, (double) ri, rhr0);
     }
-  double in1[3] = { rr0, 0.0, rhr0 }, out1[3];
+  double in1[3] = { rr0, 0.0, rhr0 };
   if (RR && !zero_x)
     for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
       in1[1] = fma ((double) x[i], (double) x[i], in1[1]);
-  team_sum<3> (cl, in1, out1);
-  if (threadIdx.x == 0)
-    sc.a = norm_ref > 0.0 ? norm_ref : sqrt (out1[0]);
-  __syncthreads ();
-  const double nb = sc.a;
-  double rho = out1[2], rr = out1[0]; // rho = (rh, r0), rh = r0 unless perturbed
-  double mark_rr = out1[0];           // best (r, r) at the last halving
-  int mark_it = 0;
-  double rho_prev = 1.0, alpha = 1.0, omega = 1.0;
-  // Team-uniform (every thread holds the same rr), so no broadcast needed.
-  double best_rr = rr, snap_rr = INFINITY;
-  // Replacement bound: kept by thread 0 only, which takes every scalar
-  // decision (nn = (x', x') of the last iteration, or the base's (g, g) at
-  // the start and after a replacement, when reset says so).
+  const double *sums = team_sum<3> (cl, turn, in1);
   constexpr double eps = 0x1p-53;
-  double dev = 0.0, dev0 = 0.0, nr_prev = 0.0, nn = out1[1];
-  bool reset = true;
+  if (threadIdx.x == 0)
+    {
+      const double rr = sums[0];
+      sc.nb = norm_ref > 0.0 ? norm_ref : sqrt (rr);
+      sc.rr = sc.best_rr = rr;
+      sc.rho = sums[2]; // (rh, r0), rh = r0 unless perturbed
+      sc.nn = sums[1];
+      sc.rho_prev = sc.alpha = sc.omega = 1.0;
+      sc.blow_rr = 1e16 * rr;
+      sc.mark_4th = 0.25 * rr;
+      sc.snap_rr = sc.snap_4th = INFINITY;
+      sc.mark_it = 0;
+      sc.reset = 1;
+    }
+  __syncthreads ();
+  const unsigned step = blockDim.x >= 128 ? 32 : 1; // one warp to a divide, if there are four
+  // a breakdown inside an iteration (thread 0): the residual reached, and
+  // whether the copy is better
+  auto mid_breakdown = [&] () {
+    sc.restore = snap && sc.snap_rr < INFINITY && !(sc.rr <= sc.snap_rr);
+    sc.rel = sc.nb > 0.0 ? sqrt (sc.restore ? sc.snap_rr : sc.rr) / sc.nb : 0.0;
+  };
   for (;;)
     {
-      if (rr < best_rr)
-        best_rr = rr;
-      if (best_rr <= 0.25 * mark_rr)
-        {
-          mark_rr = best_rr;
-          mark_it = o.iters;
-        }
-      if (snap && rr < 0.25 * snap_rr)
-        {
-          for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
-            snap[i] = RR ? x[i] + xp[i] : x[i];
-          snap_rr = rr;
-        }
       // convergence, limits and beta (gpu/bicgstab.cu:451, :512)
+      if (threadIdx.x == 0)
+        sc.rho_ratio = sc.rho / sc.rho_prev;
+      else if (threadIdx.x == step)
+        sc.step_ratio = sc.alpha / sc.omega;
+      else if (threadIdx.x == 2 * step)
+        sc.nr = sqrt (sc.rr);
+      else if (RR && threadIdx.x == 3 * step)
+        sc.root_nn = sqrt (sc.nn);
       __syncthreads ();
       if (threadIdx.x == 0)
         {
+          const double nr = sc.nr, rr = sc.rr, rho = sc.rho, nb = sc.nb;
+          if (less_abs (rr, sc.best_rr))
+            {
+              sc.best_rr = rr;
+              sc.blow_rr = 1e16 * rr;
+            }
+          if (!less_abs (sc.mark_4th, sc.best_rr))
+            {
+              sc.mark_4th = 0.25 * sc.best_rr;
+              sc.mark_it = o.iters;
+            }
+          sc.snap = snap && less_abs (rr, sc.snap_4th);
+          if (sc.snap)
+            {
+              sc.snap_rr = rr;
+              sc.snap_4th = 0.25 * rr;
+            }
           int st = 0;
           double beta = 0.0;
-          if (nb == 0.0 || sqrt (rr) < tol * nb)
+          if (is_zero (nb) || less_abs (nr, tol * nb))
             st = 1;
           else if (o.iters >= max_it)
             st = 2;
-          else if (stall > 0 && o.iters - mark_it >= stall)
+          else if (stall > 0 && o.iters - sc.mark_it >= stall)
             st = 4;
-          else if (rho == 0.0 || omega == 0.0 || !isfinite (rho) || !(rr <= 1e16 * best_rr))
+          else if (is_zero (rho) || is_zero (sc.omega) || !is_finite (rho) || !is_finite (rr)
+                   || less_abs (sc.blow_rr, rr))
             st = 3;
           else
             {
-              beta = rho / rho_prev * alpha / omega;
-              if (!isfinite (beta))
+              beta = sc.rho_ratio * sc.step_ratio;
+              if (!is_finite (beta))
                 st = 3;
             }
           int rep = 0;
           if (RR && st == 0)
             {
-              const double nr = sqrt (rr);
-              if (reset)
-                dev = dev0 = eps * (cA * sqrt (nn) + nr);
+              const double limit = kReplaceThreshold * nr;
+              if (sc.reset)
+                {
+                  sc.dev = eps * (cA * sc.root_nn + nr);
+                  sc.dev_min = 1.1 * sc.dev;
+                }
               else
                 {
-                  const double dnew = dev + eps * (cA * sqrt (nn) + nr);
-                  rep = dev <= kReplaceThreshold * nr_prev && dnew > kReplaceThreshold * nr && dnew > 1.1 * dev0;
-                  dev = dnew;
+                  const double dnew = fma (eps, cA * sc.root_nn + nr, sc.dev);
+                  rep = !less_abs (sc.limit_prev, sc.dev) && less_abs (limit, dnew) && less_abs (sc.dev_min, dnew);
+                  sc.dev = dnew;
                 }
-              nr_prev = nr;
-              reset = rep;
+              sc.limit_prev = limit;
+              sc.reset = rep;
             }
-          sc.b = beta;
-          sc.c = nb > 0.0 ? sqrt (rr) / nb : 0.0;
+          sc.beta = beta;
+          if (st)
+            {
+              sc.restore = snap && st != 1 && sc.snap_rr < INFINITY && !(rr <= sc.snap_rr);
+              sc.rel = nb > 0.0 ? (sc.restore ? sqrt (sc.snap_rr) : nr) / nb : 0.0;
+            }
           sc.status = st;
           sc.rep = rep;
         }
       __syncthreads ();
+      if (sc.snap)
+        for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
+          snap[i] = RR ? x[i] + xp[i] : x[i];
       if (sc.status)
         {
           o.status = sc.status;
-          o.rec_rel = sc.c;
+          o.rec_rel = sc.rel;
           break;
         }
       if constexpr (RR)
@@ -452,90 +552,143 @@ __device__ SolveOut team_bicgstab (cg::cluster_group &cl, const TeamSys<T> &S, c
             cl.sync ();
             EpiReplaceT er{ bt, S.r, S.rh };
             Op::run (S, ix, x, S.t, er);
-            double d4[3] = { er.rhr, er.rr, gg }, nr4[3];
-            team_sum<3> (cl, d4, nr4);
-            rho = nr4[0];
-            rr = nr4[1];
-            nn = nr4[2];
+            double d4[3] = { er.rhr, er.rr, gg };
+            sums = team_sum<3> (cl, turn, d4);
+            if (threadIdx.x == 0)
+              {
+                sc.rho = sums[0];
+                sc.rr = sums[1];
+                sc.nn = sums[2];
+              }
+            __syncthreads ();
             if (reps)
               (*reps)++;
             continue; // convergence is checked on the replaced residual
           }
-      const T tb = (T) sc.b, tw = (T) omega;
-      for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
-        S.p[i] = S.r[i] + tb * (S.p[i] - tw * S.v[i]);
+      const T tb = (T) sc.beta, tw = (T) sc.omega;
+      for (int64_t i0 = ix.elem0; i0 < S.n; i0 += kRows * ix.elem_stride)
+        {
+          T rv[kRows], pv[kRows], vv[kRows];
+#pragma unroll
+          for (int u = 0; u < kRows; u++)
+            {
+              const int64_t iu = i0 + u * ix.elem_stride, i = iu < S.n ? iu : i0;
+              rv[u] = S.r[i];
+              pv[u] = S.p[i];
+              vv[u] = S.v[i];
+            }
+#pragma unroll
+          for (int u = 0; u < kRows; u++)
+            if (const int64_t i = i0 + u * ix.elem_stride; i < S.n)
+              S.p[i] = rv[u] + tb * (pv[u] - tw * vv[u]);
+        }
       cl.sync ();
       EpiDotT<T> e2{ S.rh };
       Op::run (S, ix, S.p, S.v, e2);
-      double d1[1] = { e2.acc }, rhv[1];
-      team_sum<1> (cl, d1, rhv);
+      double d1[1] = { e2.acc };
+      sums = team_sum<1> (cl, turn, d1);
       if (threadIdx.x == 0)
         {
-          sc.a = rho / rhv[0];
-          sc.status = (rhv[0] == 0.0 || !isfinite (sc.a)) ? 3 : 0;
+          const double a = sc.rho / sums[0];
+          sc.alpha = a;
+          sc.status = (is_zero (sums[0]) || !is_finite (a)) ? 3 : 0;
+          if (sc.status)
+            mid_breakdown ();
         }
       __syncthreads ();
       if (sc.status)
         {
           o.status = 3;
-          o.rec_rel = nb > 0.0 ? sqrt (rr) / nb : 0.0;
+          o.rec_rel = sc.rel;
           break;
         }
-      alpha = sc.a;
-      const T ta = (T) alpha;
-      for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
-        S.s[i] = S.r[i] - ta * S.v[i];
+      const T ta = (T) sc.alpha;
+      for (int64_t i0 = ix.elem0; i0 < S.n; i0 += kRows * ix.elem_stride)
+        {
+          T rv[kRows], vv[kRows];
+#pragma unroll
+          for (int u = 0; u < kRows; u++)
+            {
+              const int64_t iu = i0 + u * ix.elem_stride, i = iu < S.n ? iu : i0;
+              rv[u] = S.r[i];
+              vv[u] = S.v[i];
+            }
+#pragma unroll
+          for (int u = 0; u < kRows; u++)
+            if (const int64_t i = i0 + u * ix.elem_stride; i < S.n)
+              S.s[i] = rv[u] - ta * vv[u];
+        }
       cl.sync ();
       EpiTST<T> e4{ S.s };
       Op::run (S, ix, S.s, S.t, e4);
-      double d2[2] = { e4.ts, e4.tt }, tst[2];
-      team_sum<2> (cl, d2, tst);
+      double d2[2] = { e4.ts, e4.tt };
+      sums = team_sum<2> (cl, turn, d2);
       if (threadIdx.x == 0)
         {
-          const double w = tst[1] != 0.0 ? tst[0] / tst[1] : 0.0;
-          sc.a = w;
-          sc.status = isfinite (w) ? 0 : 3;
+          const double w = is_zero (sums[1]) ? 0.0 : sums[0] / sums[1];
+          sc.omega = w;
+          sc.status = is_finite (w) ? 0 : 3;
+          if (sc.status)
+            mid_breakdown ();
         }
       __syncthreads ();
       if (sc.status)
         {
           o.status = 3;
-          o.rec_rel = nb > 0.0 ? sqrt (rr) / nb : 0.0;
+          o.rec_rel = sc.rel;
           break;
         }
-      omega = sc.a;
-      const T tw2 = (T) omega;
+      const T tw2 = (T) sc.omega;
       double rhr = 0.0, rrn = 0.0, xx = 0.0;
       T *xu = RR ? xp : x; // the vector the iteration updates
-      for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
+      constexpr int kUp = kRows / 2;
+      for (int64_t i0 = ix.elem0; i0 < S.n; i0 += kUp * ix.elem_stride)
         {
-          const T xn = xu[i] + ta * S.p[i] + tw2 * S.s[i];
-          xu[i] = xn;
-          const T ri = S.s[i] - tw2 * S.t[i];
-          S.r[i] = ri;
-          rhr = fma ((double) S.rh[i], (double) ri, rhr);
-          rrn = fma ((double) ri, (double) ri, rrn);
-          if (RR)
-            xx = fma ((double) xn, (double) xn, xx);
+          T xv[kUp], pv[kUp], sv[kUp], tv[kUp], hv[kUp];
+#pragma unroll
+          for (int u = 0; u < kUp; u++)
+            {
+              const int64_t iu = i0 + u * ix.elem_stride, i = iu < S.n ? iu : i0;
+              xv[u] = xu[i];
+              pv[u] = S.p[i];
+              sv[u] = S.s[i];
+              tv[u] = S.t[i];
+              hv[u] = S.rh[i];
+            }
+#pragma unroll
+          for (int u = 0; u < kUp; u++)
+            if (const int64_t i = i0 + u * ix.elem_stride; i < S.n)
+              {
+                const T xn = xv[u] + ta * pv[u] + tw2 * sv[u];
+                xu[i] = xn;
+                const T ri = sv[u] - tw2 * tv[u];
+                S.r[i] = ri;
+                const double rd = widen (ri);
+                rhr = fma (widen (hv[u]), rd, rhr);
+                rrn = fma (rd, rd, rrn);
+                if (RR)
+                  xx = fma (widen (xn), widen (xn), xx);
+              }
         }
-      double d3[3] = { rhr, rrn, xx }, nx[3];
-      team_sum<3> (cl, d3, nx);
-      rho_prev = rho;
-      rho = nx[0];
-      rr = nx[1];
-      nn = nx[2];
+      double d3[3] = { rhr, rrn, xx };
+      sums = team_sum<3> (cl, turn, d3);
+      if (threadIdx.x == 0)
+        {
+          sc.rho_prev = sc.rho;
+          sc.rho = sums[0];
+          sc.rr = sums[1];
+          sc.nn = sums[2];
+        }
+      __syncthreads ();
       o.iters++;
     }
-  if (snap && o.status != 1 && snap_rr < INFINITY && !(rr <= snap_rr))
-    {
-      for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
-        {
-          x[i] = snap[i];
-          if (RR)
-            xp[i] = 0;
-        }
-      o.rec_rel = nb > 0.0 ? sqrt (snap_rr) / nb : 0.0;
-    }
+  if (sc.restore)
+    for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
+      {
+        x[i] = snap[i];
+        if (RR)
+          xp[i] = 0;
+      }
   if (RR)
     for (int64_t i = ix.elem0; i < S.n; i += ix.elem_stride)
       {
@@ -548,17 +701,17 @@ __device__ SolveOut team_bicgstab (cg::cluster_group &cl, const TeamSys<T> &S, c
 
 // r = b - A x in FP64 over the team; returns (||r||^2, ||b||^2).
 template <int OP>
-__device__ void team_residual (cg::cluster_group &cl, const TeamSys<double> &S, const double *b, const double *x,
+__device__ void team_residual (cg::cluster_group &cl, int &turn, const TeamSys<double> &S, const double *b, const double *x,
                                double *r, double &rr, double &bb)
 {
   using Op = TeamOp<double, OP>;
   const TeamIdx ix = team_index<Op::G> (cl);
   EpiResid e{ b, r };
   Op::run (S, ix, x, S.t, e); // y lands in t (scratch)
-  double d[2] = { e.rr, e.bb }, out[2];
-  team_sum<2> (cl, d, out);
-  rr = out[0];
-  bb = out[1];
+  double d[2] = { e.rr, e.bb };
+  const double *sums = team_sum<2> (cl, turn, d);
+  rr = sums[0];
+  bb = sums[1];
 }
 
 struct Fp64Result
@@ -576,7 +729,7 @@ struct Fp64Result
 // attainable accuracy a restart can leave x worse, so the best iterate is
 // kept (xb) and restored.
 template <int OP>
-__device__ Fp64Result fp64_restarted (cg::cluster_group &cl, const TeamSys<double> &S64, const BatchDesc &D,
+__device__ Fp64Result fp64_restarted (cg::cluster_group &cl, int &turn, const TeamSys<double> &S64, const BatchDesc &D,
                                       const BatchParams &P, bool first, int budget, double norm_b, double *r64,
                                       double cA)
 {
@@ -591,13 +744,13 @@ __device__ Fp64Result fp64_restarted (cg::cluster_group &cl, const TeamSys<doubl
   bool shadow = false;   // restart after a breakdown: perturbed shadow residual
   for (;;)
     {
-      const SolveOut o = team_bicgstab<double, OP, true> (cl, S64, first ? D.b : r64, D.x, first, target,
+      const SolveOut o = team_bicgstab<double, OP, true> (cl, turn, S64, first ? D.b : r64, D.x, first, target,
                                                           budget - f.iters, norm_b, snap, 0, D.b, xp, cA,
                                                           &f.replacements, shadow);
       shadow = o.status == 3;
       f.iters += o.iters;
       double rr, bb;
-      team_residual<OP> (cl, S64, D.b, D.x, r64, rr, bb);
+      team_residual<OP> (cl, turn, S64, D.b, D.x, r64, rr, bb);
       if (threadIdx.x == 0)
         {
           sh_rel = bb > 0 ? sqrt (rr / bb) : 0.0;
@@ -647,7 +800,7 @@ __device__ Fp64Result fp64_restarted (cg::cluster_group &cl, const TeamSys<doubl
 }
 
 template <int PREC, int OP>
-__device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const BatchParams &P, BatchOut &res)
+__device__ void solve_system (cg::cluster_group &cl, int &turn, const BatchDesc &D, const BatchParams &P, BatchOut &res)
 {
   TeamSys<double> S64{ D.nbr, D.bs, D.n, D.rp, D.cols, D.vals64,
                        D.w64, D.w64 + D.n, D.w64 + 2 * D.n, D.w64 + 3 * D.n, D.w64 + 4 * D.n, D.w64 + 5 * D.n };
@@ -666,7 +819,7 @@ __device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const B
       for (int64_t i = ix.elem0; i < D.n; i += ix.elem_stride)
         b32[i] = (float) D.b[i];
       cl.sync ();
-      const SolveOut o = team_bicgstab<float, OP> (cl, S32, b32, x32, true, P.tol, P.max_it, -1.0);
+      const SolveOut o = team_bicgstab<float, OP> (cl, turn, S32, b32, x32, true, P.tol, P.max_it, -1.0);
       for (int64_t i = ix.elem0; i < D.n; i += ix.elem_stride)
         D.x[i] = (double) x32[i];
       cl.sync ();
@@ -674,12 +827,12 @@ __device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const B
       status = o.status;
       rec = o.rec_rel;
       double rr, bb;
-      team_residual<OP> (cl, S64, D.b, D.x, r64, rr, bb);
+      team_residual<OP> (cl, turn, S64, D.b, D.x, r64, rr, bb);
       rel = bb > 0 ? sqrt (rr / bb) : 0.0;
     }
   else if constexpr (PREC == BMFP_SOLVE_FP64)
     {
-      const Fp64Result f = fp64_restarted<OP> (cl, S64, D, P, true, P.max_it, -1.0, r64, cA);
+      const Fp64Result f = fp64_restarted<OP> (cl, turn, S64, D, P, true, P.max_it, -1.0, r64, cA);
       iters64 = f.iters;
       status = f.status;
       restarts = f.restarts;
@@ -702,7 +855,7 @@ __device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const B
       for (int k = 0;; k++)
         {
           double rr, bb;
-          team_residual<OP> (cl, S64, D.b, D.x, r64, rr, bb);
+          team_residual<OP> (cl, turn, S64, D.b, D.x, r64, rr, bb);
           if (threadIdx.x == 0)
             {
               sh_rel = bb > 0 ? sqrt (rr / bb) : 0.0;
@@ -733,7 +886,7 @@ __device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const B
               // exactly as the FP64 solve does (same ||b||, same bits).
               const bool fresh = rel > 1e-2;
               const Fp64Result f
-                = fp64_restarted<OP> (cl, S64, D, P, fresh, P.max_it - iters32, fresh ? -1.0 : nb, r64, cA);
+                = fp64_restarted<OP> (cl, turn, S64, D, P, fresh, P.max_it - iters32, fresh ? -1.0 : nb, r64, cA);
               iters64 += f.iters;
               status = f.status;
               restarts = f.restarts;
@@ -749,7 +902,7 @@ __device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const B
             r32[i] = (float) (r64[i] * inv);
           cl.sync ();
           const int cap = min (P.inner_max, P.max_it - iters32 - iters64);
-          const SolveOut o = team_bicgstab<float, OP> (cl, S32, r32, x32, true, P.inner_tol, cap, -1.0,
+          const SolveOut o = team_bicgstab<float, OP> (cl, turn, S32, r32, x32, true, P.inner_tol, cap, -1.0,
                                                        nullptr, P.inner_stall);
           iters32 += o.iters;
           refinements = k + 1;
@@ -792,15 +945,19 @@ __device__ void solve_system (cg::cluster_group &cl, const BatchDesc &D, const B
 }
 
 // Two CTAs of 512 threads per SM (64 registers a thread, some spilled): two
-// teams share each SM's FP64 pipe and hide each other's latency. On the
-// uneven elasticity batch (FP64, cluster 8 x 512) 0.66 s against 0.92 s at
-// one CTA per SM and 128 registers, and the best configuration of either
-// bound: 0.66 against 0.76 s.
+// teams share each SM's FP64 pipe and hide each other's latency. What bounds
+// it: the round trips and barriers of a team's iteration (a few rows per
+// thread), not bandwidth. 256 uneven systems of K + 0.01 I (3.2 M rows), one
+// launch, ms for clusters 4 x 512, 8 x 256, 8 x 512: mixed 42.8, 42.4, 39.4
+// (before the integer team sums, the scalars in shared memory and the loads
+// ahead of the vector updates 53.7, 53.9, 62.7); FP64 91.7, 82.8, 72.7
+// (102.8, 99.5, 93.3).
 template <int PREC, int OP>
 __global__ void __launch_bounds__ (512, 2) batch_kernel (BatchParams P)
 {
   cg::cluster_group cl = cg::this_cluster ();
   __shared__ int sh_sys;
+  int turn = 0; // team_sum's
   for (;;)
     {
       if (cl.block_rank () == 0 && threadIdx.x == 0)
@@ -812,7 +969,7 @@ __global__ void __launch_bounds__ (512, 2) batch_kernel (BatchParams P)
         break;
       const int sys = P.order[k];
       const BatchDesc D = P.desc[sys];
-      solve_system<PREC, OP> (cl, D, P, P.out[sys]);
+      solve_system<PREC, OP> (cl, turn, D, P, P.out[sys]);
     }
 }
 

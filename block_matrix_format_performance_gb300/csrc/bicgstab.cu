@@ -48,6 +48,7 @@
 // and a solve finishes with a true-residual check b - A x (restarting from
 // the true residual when the recursive one has drifted below the tolerance
 // first).
+#include "reduce.cuh"
 #include "solver.h"
 #include "spmv_core.cuh"
 
@@ -62,6 +63,8 @@
 
 namespace bmfp
 {
+using namespace reduce;
+
 namespace
 {
 constexpr int kThreads = 256;
@@ -100,75 +103,6 @@ template <typename T> struct Args
   const T *svals;
   int nslices;
 };
-
-// Sum over a warp, the same on every lane: each value's mantissa shifted to
-// the largest exponent of the warp (five guard bits: more than the FP64 adds
-// of a butterfly keep), the integers added exactly in three limbs by redux,
-// one rounding (to nearest, halves away from zero) where the result is put
-// together. A butterfly's five dependent warp-wide FP64 adds take 600 cycles
-// on GB300, whose FP64 pipe starts one warp's instruction per 64 cycles and SM
-// quarter, and keep that pipe busy throughout; this runs on the integer pipes.
-// Zeros, subnormals, infinities and NaN go to the butterfly.
-// NK values at a time: their chains of redux run side by side.
-template <int NK> __device__ __forceinline__ void warp_sums (const double (&v)[NK], double (&out)[NK])
-{
-  constexpr unsigned kAll = 0xffffffffu;
-  int top[NK];
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    top[k] = (int) __reduce_max_sync (kAll, (unsigned) ((__double2hiint (v[k]) >> 20) & 0x7ff));
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    {
-      const long long bits = __double_as_longlong (v[k]);
-      const int ex = (int) ((bits >> 52) & 0x7ff);
-      const int d = top[k] - ex;
-      long long m = ex ? ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 5 : 0;
-      m = d < 58 ? (m + ((1ll << d) >> 1)) >> d : 0;
-      if (bits < 0)
-        m = -m;
-      const unsigned lo = __reduce_add_sync (kAll, (unsigned) (m & 0xfffff));
-      const unsigned mid = __reduce_add_sync (kAll, (unsigned) ((m >> 20) & 0xfffff));
-      const int hi = __reduce_add_sync (kAll, (int) (m >> 40));
-      const long long sum = ((long long) hi << 40) + ((long long) mid << 20) + lo;
-      unsigned long long u = (unsigned long long) (sum < 0 ? -sum : sum);
-      const int lz = __clzll ((long long) u);
-      u <<= lz & 63;
-      const unsigned long long man = (u >> 11) + ((u >> 10) & 1); // 2^52 .. 2^53
-      const unsigned long long r = ((unsigned long long) (top[k] + 5 - lz) << 52) + man;
-      out[k] = __longlong_as_double (sum ? (long long) (r | (sum < 0 ? 1ull << 63 : 0)) : 0);
-    }
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    if (top[k] < 64 || top[k] > 2047 - 64)
-      {
-        double a = v[k];
-        if (__any_sync (kAll, (__double_as_longlong (a) << 1) != 0))
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1)
-            a += __shfl_xor_sync (kAll, a, off);
-        out[k] = a;
-      }
-}
-
-__device__ __forceinline__ double warp_sum (double v)
-{
-  const double in[1] = { v };
-  double out[1];
-  warp_sums<1> (in, out);
-  return out[0];
-}
-
-// Tests of doubles on the integer pipes (a DSETP costs what a DFMA does).
-__device__ __forceinline__ bool is_zero (double v) { return (__double_as_longlong (v) << 1) == 0; }
-__device__ __forceinline__ bool is_finite (double v) { return ((__double2hiint (v) >> 20) & 0x7ff) != 0x7ff; }
-// a < b for a and b non-negative, infinite or NaN (false then).
-__device__ __forceinline__ bool less_abs (double a, double b)
-{
-  const unsigned long long ua = (unsigned long long) __double_as_longlong (a),
-                           ub = (unsigned long long) __double_as_longlong (b);
-  return ua < ub && ub <= 0x7ff0000000000000ull;
-}
 
 // done and rep_now in one load. Both are written by earlier kernels (done
 // also by block 0 of phases 1, 3 and 5, in cases where every block of that

@@ -69,6 +69,32 @@ def test_fp64_batch_converges_and_matches_single_solver(lib, cuda, config):
     assert misses <= 1
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("config", [(1, 64), (2, 64), (8, 64), (1, 128), (2, 192), (8, 448), (1, 512)])
+def test_every_team_shape_solves(lib, cuda, config, precision):
+    """Teams with fewer warps than sums and than side-by-side divides (64
+    threads), warp counts that are no power of two, one CTA and the largest
+    cluster; systems smaller than a team and with rows left over. FP32 with a
+    right-hand side at 1e-30: its dot products (1e-60) need FP64's range."""
+    systems = []
+    for nx, ny in ((2, 2), (20, 5), (33, 9), (64, 16)):
+        rp, c, v, rhs = bm.gen_q4_elasticity(nx, ny)
+        rows = np.repeat(np.arange(nx * ny), np.diff(rp))
+        v.reshape(-1, 2, 2)[c == rows] += 0.05 * np.eye(2)
+        rhs = np.random.default_rng(nx).uniform(-1, 1, rhs.size)
+        systems.append((rp, c, v, rhs * (1e-30 if precision == "fp32" else 1.0), 2))
+    tol = 1e-5 if precision == "fp32" else 1e-10
+    xs, infos = run_batch(systems, precision, config, tol=tol)
+    for (rp, c, v, rhs, bs), x, info in zip(systems, xs, infos):
+        K = csr_of(rp, c, v, bs)
+        rel = np.linalg.norm((rhs - K @ x) / np.linalg.norm(rhs))
+        # FP32: the recursive residual meets the tolerance; the true one may
+        # stand a rounding of x (2^-24 ||K|| ||x|| / ||b||, below 2e-5 here) above it
+        assert rel < (tol if precision != "fp32" else 4e-5), (rel, info)
+        if precision != "fp32":
+            assert info["status"] == bm.SUCCESS, info
+
+
 def test_result_is_bitwise_the_same_alone_and_in_the_mix(lib, cuda):
     systems = q4_systems(GRIDS)
     xs_mix, inf_mix = run_batch(systems, "fp64", (4, 256))
