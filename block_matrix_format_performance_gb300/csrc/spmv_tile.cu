@@ -15,7 +15,7 @@
 // (50-70 % busy) and the latency of x; FP32, the latency of the two round trips
 // a tile makes (values and columns, then x). us, before (warp per block row)
 // and now: rows of 0-15 blocks, 150 000 block rows, bs 3 FP64 77.7 -> 35.2,
-// FP32 26.2 -> 21.1; 50 000 block rows of 6 blocks, bs 12 FP32 40.4 -> 36.9,
+// FP32 26.2 -> 21.1; 50 000 block rows of 6 blocks, bs 12 FP32 40.4 -> 34.5,
 // FP64 102 -> 97, bs 17 FP64 279 -> 202, FP32 96 -> 69, bs 24 FP64 558 -> 411.
 #include "device_common.cuh"
 #include "internal.h"
@@ -104,10 +104,13 @@ struct TilePlan
 };
 
 // Blocks whose x segments a thread has in flight at once.
-constexpr int blocks_in_flight (int bs) { return bs == 1 ? 5 : bs <= 3 ? 3 : bs <= 6 ? 2 : 1; }
+constexpr int blocks_in_flight (int bs, int bytes)
+{
+  return bs <= 3 ? 3 : bs <= 6 ? 2 : bs <= 12 && bytes == 4 ? 2 : 1;
+}
 
 template <typename T, int BSC, int V, bool PAD>
-__global__ void __launch_bounds__ (kThreads, 8)
+__global__ void __launch_bounds__ (kThreads, BSC == 3 ? 10 : 8)
   tile_kernel (int nbr, int bs_rt, TilePlan P, const int *__restrict__ row_ptr, const int *__restrict__ cols,
                const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
 {
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__ (kThreads, 8)
             };
             if constexpr (BSC != 0)
               {
-                constexpr int UB = blocks_in_flight (BSC);
+                constexpr int UB = blocks_in_flight (BSC, sizeof (T));
                 while (b < be)
                   {
                     Pack<T, V> xv[UB][BSC / V];
@@ -213,19 +216,31 @@ __global__ void __launch_bounds__ (kThreads, 8)
                           for (int c = 0; c < BSC / V; c++)
                             xv[u][c] = ld_x<T, V> (xb + c * V);
                         }
+                    // the lines of two long-lined blocks before the first
+                    // flush: the branches in done () would keep them apart
+                    constexpr bool kAhead = UB > 1 && BSC > 6;
+                    Pack<T, V> av[UB][BSC / V];
+                    auto lines = [&] (int u, int at_block) {
+                      const int line = off + at_block * E + r * BSC;
+#pragma unroll
+                      for (int c = 0; c < BSC / V; c++)
+                        av[u][c] = ld_s<T, V> (sv + at<T, PAD> (line + c * V));
+                    };
+                    if (kAhead)
+#pragma unroll
+                      for (int u = 0; u < UB; u++)
+                        lines (u, b + min (u, left - 1));
 #pragma unroll
                     for (int u = 0; u < UB; u++)
                       if (u == 0 || u < left)
                         {
-                          const int line = off + b * E + r * BSC;
+                          if (!kAhead)
+                            lines (u, b);
 #pragma unroll
                           for (int c = 0; c < BSC / V; c++)
-                            {
-                              const Pack<T, V> av = ld_s<T, V> (sv + at<T, PAD> (line + c * V));
 #pragma unroll
-                              for (int k = 0; k < V; k++)
-                                acc = fma (av.v[k], xv[u][c].v[k], acc);
-                            }
+                            for (int k = 0; k < V; k++)
+                              acc = fma (av[u][c].v[k], xv[u][c].v[k], acc);
                           done ();
                         }
                   }
@@ -320,7 +335,7 @@ int tile_typed (int nbr, int bs, int64_t nnzb, const int *rp, const int *c, cons
   // whose partial sums take more room): eight CTAs an SM hide one another's
   // copies. Measured at 12 to 52 KB and with 256 threads per CTA; larger tiles
   // and room kept for rows above the average were slower.
-  const double room = (bs <= 5 ? 20 : 24) * 1024;
+  const double room = (bs <= (sizeof (T) == 4 ? 8 : 5) ? 20 : 24) * 1024;
   TilePlan P{};
   const int slots = kThreads / bs;
   P.chunk = std::max (1, (int) (room / (block * slots) + 0.5));
