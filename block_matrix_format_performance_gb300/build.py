@@ -27,6 +27,7 @@ LIB = os.path.join(PKG, "libbmfp.so")
 SOURCES = [
     "spmv_native.cu",
     "spmv_tile.cu",
+    "spmv_ring.cu",
     "spmv_variants.cu",
     "spmv_host.cpp",
     "peaks.cu",

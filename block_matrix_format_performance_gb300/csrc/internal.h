@@ -46,6 +46,11 @@ int spmv_native_csr (int dtype, int n_rows, int64_t nnz, const int *row_ptr, con
 // the matrix has too few tiles to fill the GPU.
 int spmv_tile (int dtype, int n_block_rows, int bs, int64_t nnzb, const int *row_ptr, const int *cols,
                const void *vals, const void *x, void *y, bool *took, cudaStream_t stream);
+// FP64 product for bs 16 and 32 by per-warp rings of staged blocks (vals and x
+// 16-byte aligned), and whether it is the faster one.
+bool spmv_ring_wins (int bs, int n_block_rows);
+int spmv_ring (int n_block_rows, int bs, const int *row_ptr, const int *cols, const double *vals, const double *x,
+               double *y, cudaStream_t stream);
 int spmv_reference_variant (int dtype, int variant, int n_rows, int n_cols, int bs, int64_t nnz,
                             const int *row_ptr, const int *cols, const void *vals, const void *x,
                             void *y, cudaStream_t stream);

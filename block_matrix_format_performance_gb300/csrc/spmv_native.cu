@@ -16,6 +16,8 @@
 //    and a fixed set of rows per phase (chunk < block). Partial row sums are
 //    combined with xor-shuffles over exactly the lane bits that vary the
 //    column, so the reduction costs log2 steps and no shared memory.
+//  * a ring of staged blocks per warp (spmv_ring.cu: FP64 at bs 16 and 32, the
+//    default lanes).
 //  * row tiles (spmv_tile.cu: bs <= 32 that is no power of two, e.g. 3 for
 //    frame elements, from a few hundred tiles up).
 //  * bcsr_tpr_kernel (any bs <= 32, small or misaligned): a warp owns
@@ -273,6 +275,9 @@ int native_bcsr_typed (int nbr, int bs, int64_t nnzb, const int *rp, const int *
       const bool ok = (reinterpret_cast<uintptr_t> (v) | reinterpret_cast<uintptr_t> (x)) % 16 == 0;
       if (lanes == BMFP_LANES_ROW_OWNER && (!ok || bs < 4))
         lanes = 0; // misaligned views: the scalar-load kernel below
+      if constexpr (sizeof (T) == 8)
+        if (ok && spmv_ring_wins (bs, nbr))
+          return spmv_ring (nbr, bs, rp, c, v, x, y, s);
     }
   if (lanes == BMFP_LANES_ROW_OWNER)
     {

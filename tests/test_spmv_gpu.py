@@ -241,6 +241,38 @@ def test_row_tiles(lib, orc, cuda, bs, kind, dtype):
         assert np.all(np.abs(y[:n] - orc.bcsr_spmv(rp, c, v, bs, xf[off:])) <= tol)
 
 
+@pytest.mark.parametrize("kind", ["uneven", "empty tail", "one row", "no blocks"])
+@pytest.mark.parametrize("nbr", [1, 7, 1216, 1217, 2432, 2433, 4864, 4865])
+@pytest.mark.parametrize("bs", [16, 32])
+def test_staged_rings(lib, orc, cuda, bs, nbr, kind):
+    """FP64 at bs 16 and 32 around its numbers of rows per group: empty rows at
+    both ends and in stretches, all blocks in one row, no blocks at all."""
+    import torch
+    rng = np.random.default_rng(nbr + bs)
+    counts = rng.integers(0, 6, nbr)
+    counts[[0, nbr - 1]] = 0
+    if kind == "empty tail":
+        counts[nbr // 8:] = 0
+    elif kind == "one row":
+        counts[:] = 0
+        counts[nbr // 3] = 50
+    elif kind == "no blocks":
+        counts[:] = 0
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    nnzb, nbc = int(rp[-1]), 300
+    c = rng.integers(0, nbc, nnzb).astype(np.int32)
+    v, x = rng.uniform(-1, 1, nnzb * bs * bs), rng.uniform(-1, 1, nbc * bs)
+    n = nbr * bs
+    d_y = torch.full((n + GUARD,), float("nan"), dtype=torch.float64, device="cuda")
+    d_c, d_v = (dev(c), dev(v)) if nnzb else (dev(np.zeros(1, np.int32)), dev(np.zeros(bs * bs)))
+    bm.bcsr_spmv(bm.BCSR_NATIVE, dev(rp), d_c, d_v, dev(x), d_y, bs, nbc)
+    y = d_y.cpu().numpy()
+    assert np.isnan(y[n:]).all()
+    crp, cc, cv = orc.bcsr_to_csr(rp, c, v, bs)
+    tol = spmv_tolerance(orc, crp, cc, cv, x, np.float64)
+    assert np.all(np.abs(y[:n] - orc.bcsr_spmv(rp, c, v, bs, x)) <= tol)
+
+
 def test_empty_and_zero_block_matrices(lib, orc, cuda):
     import torch
     # no block rows at all: a valid no-op
