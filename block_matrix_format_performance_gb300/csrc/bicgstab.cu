@@ -1758,8 +1758,8 @@ int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
   const int64_t vectors = 7 * S * P.rows;
   if (!coop || vectors > most)
     return BMFP_SUCCESS;
-  const size_t o_flags = sizeof (unsigned long long) * 2 * kSlotKinds * 2 * (size_t) P.grid;
-  const size_t o_need = (o_flags + sizeof (unsigned) * (size_t) P.grid + 15) / 16 * 16;
+  const size_t o_flags = sizeof (unsigned long long) * 2 * kSlotKinds * 2 * kCopies * (size_t) P.grid;
+  const size_t o_need = (o_flags + sizeof (unsigned) * kFlagStride * (size_t) P.grid + 15) / 16 * 16;
   BMFP_CUDA (cudaMalloc (&resident_mem_, o_need + sizeof (int2) * ((size_t) P.grid + 1)));
   resident_zero_ = o_need;
   BMFP_CUDA (cudaMemsetAsync (resident_mem_, 0, o_need + sizeof (int2) * ((size_t) P.grid + 1), s));

@@ -67,6 +67,75 @@ __device__ __forceinline__ double warp_sum (double v)
   return out[0];
 }
 
+// Sum over a warp and the M values of each of its lanes (M <= 32), as
+// warp_sums does it: 1024 terms of 58 bits take 68.
+template <int M> __device__ __forceinline__ double warp_sum_of (const double (&v)[M])
+{
+  constexpr unsigned kAll = 0xffffffffu;
+  static_assert (M <= 32, "a lane's terms fit 63 bits");
+  int ex[M], top = 0;
+#pragma unroll
+  for (int j = 0; j < M; j++)
+    {
+      ex[j] = (__double2hiint (v[j]) >> 20) & 0x7ff;
+      top = max (top, ex[j]);
+    }
+  top = (int) __reduce_max_sync (kAll, (unsigned) top);
+  if (top < 64 || top > 2047 - 64)
+    {
+      double a = v[0];
+#pragma unroll
+      for (int j = 1; j < M; j++)
+        a += v[j];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1)
+        a += __shfl_xor_sync (kAll, a, off);
+      return a;
+    }
+  long long m = 0;
+#pragma unroll
+  for (int j = 0; j < M; j++)
+    {
+      const long long bits = __double_as_longlong (v[j]);
+      const int d = top - ex[j];
+      long long a = ex[j] ? ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 5 : 0;
+      a = d < 58 ? (a + ((1ll << d) >> 1)) >> d : 0;
+      m += bits < 0 ? -a : a;
+    }
+  const unsigned lo = __reduce_add_sync (kAll, (unsigned) (m & 0xfffff));
+  const unsigned mid = __reduce_add_sync (kAll, (unsigned) ((m >> 20) & 0xfffff));
+  const int hi = __reduce_add_sync (kAll, (int) (m >> 40));
+  // in units of 2^20, and the rest
+  long long a = ((long long) hi << 20) + mid + (lo >> 20);
+  unsigned b = lo & 0xfffff;
+  const bool minus = a < 0;
+  if (minus)
+    {
+      a = -a - (b != 0);
+      b = (0x100000u - b) & 0xfffff;
+    }
+  if (a == 0 && b == 0)
+    return 0.0;
+  // normalised: bit 63 set, bits below the last place of 68 dropped
+  const int la = __clzll (a);
+  int lz; // zeros above the value's first bit in 84 bits
+  unsigned long long u;
+  if (la < 64)
+    {
+      lz = la;
+      u = la >= 20 ? ((unsigned long long) a << la) | ((unsigned long long) b << (la - 20))
+                   : ((unsigned long long) a << la) | (b >> (20 - la));
+    }
+  else
+    {
+      lz = 64 + __clz ((int) b) - 12;
+      u = (unsigned long long) b << (32 + __clz ((int) b));
+    }
+  const unsigned long long man = (u >> 11) + ((u >> 10) & 1); // 2^52 .. 2^53
+  const unsigned long long r = ((unsigned long long) (top + 5 + 20 - lz) << 52) + man;
+  return __longlong_as_double ((long long) (r | (minus ? 1ull << 63 : 0)));
+}
+
 // Tests of doubles on the integer pipes (a DSETP costs what a DFMA does).
 __device__ __forceinline__ bool is_zero (double v) { return (__double_as_longlong (v) << 1) == 0; }
 __device__ __forceinline__ bool is_finite (double v) { return ((__double2hiint (v) >> 20) & 0x7ff) != 0x7ff; }

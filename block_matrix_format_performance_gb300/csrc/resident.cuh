@@ -17,8 +17,8 @@
 //    vector goes out as it is, each CTA releases a flag behind its rows, and
 //    waits for the flags of the CTAs its columns belong to.
 //  * the three sets of dot products: each CTA writes its partial sums, every
-//    CTA reads all of them, and each derives the same scalars from the same
-//    sums in the same order. Nothing is left to a last CTA, and no counter is
+//    CTA reads all of them, a warp to a kind, and each derives the same scalars
+//    from the same sums. Nothing is left to a last CTA, and no counter is
 //    contended.
 //
 // What bounds it: small systems, the latency of five one-way trips through L2
@@ -31,14 +31,22 @@
 // us per iteration on the Q4 operator, as graphs and here: FP64 2 048 rows
 // 21.9 / 14.0, 20 000 21.5 / 17-21, 80 000 29.3 / 27.8, 500 000 66.6 / 64.2;
 // FP32 2 048 rows 19.8 / 12.6, 80 000 23.0 / 20.2, 180 000 31.4 / 22.9,
-// 500 000 39.8 / 34. Whole solves (K + 0.01 I): 200x50 FP64 4.38 -> 3.70 ms,
-// 1000x250 mixed 9.06 -> 6.72 ms.
+// 500 000 39.8 / 34. Whole solves (K + 0.01 I): 200x50 FP64 4.38 -> 2.73 ms,
+// 1000x250 mixed 9.06 -> 5.07 ms.
 #pragma once
 
 // Threads per CTA at most: products from global memory live on the loads in
 // flight, and in FP32 nine steps of them fit 64 registers.
 constexpr int resident_threads (int bytes, bool staged) { return bytes == 4 && !staged ? 1024 : 512; }
 constexpr int kSlotKinds = 3;
+// A word that all CTAs look at again and again is slow for all of them: the
+// looks queue at its line. So every CTA writes its sums in kCopies places, of
+// which a reader looks at one, and a flag has a line to itself. us per
+// iteration with one copy, 4, 8, 16 and 32: FP64 20 000 rows 19.5 / 17.4 / 16.5 /
+// 16.2 / 16.0, FP32 80 000 rows 19.8 / 18.1 / 17.7 / 17.8 / 17.9; a line to a
+// flag: FP32 500 000 rows 37.8 -> 30.8, FP64 65.8 -> 59.0.
+constexpr int kCopies = 16;
+constexpr int kFlagStride = 32; // 4-byte words
 
 using Word = unsigned long long;
 
@@ -126,11 +134,16 @@ template <class F> __device__ __forceinline__ bool wait_for (F ready)
 {
   if (ready ())
     return true;
-  const unsigned long long t0 = global_ns ();
-  unsigned polls = 0;
-  while (!ready ())
-    if ((++polls & 255u) == 0 && global_ns () - t0 > kBarrierLimitNs)
-      return false;
+  unsigned long long t0 = 0; // of the 256th look
+  for (unsigned polls = 1; !ready (); polls++)
+    if ((polls & 255u) == 0)
+      {
+        const unsigned long long now = global_ns ();
+        if (t0 == 0)
+          t0 = now;
+        else if (now - t0 > kBarrierLimitNs)
+          return false;
+      }
   return true;
 }
 
@@ -140,17 +153,17 @@ __device__ __forceinline__ bool publish (unsigned *flags, int2 need, unsigned ep
 {
   __syncthreads ();
   if (threadIdx.x == 0)
-    put_flag (flags + blockIdx.x, epoch);
+    put_flag (flags + blockIdx.x * kFlagStride, epoch);
   bool ok = true;
   for (int j = need.x + (int) threadIdx.x; j <= need.y; j += blockDim.x)
-    ok = wait_for ([&] () { return get_flag (flags + j, epoch); }) && ok;
+    ok = wait_for ([&] () { return get_flag (flags + j * kFlagStride, epoch); }) && ok;
   return __syncthreads_or (!ok) == 0;
 }
 
 // Sum NK per-thread values over the grid as exchange `epoch`, through set
 // `turn` of the words (successive sums take the two sets in turn); warp k
-// returns kind k's sum on every lane (other warps 0). False when a wait gave
-// up.
+// (k < NK <= 4 <= the CTA's warps) returns kind k's sum on every lane (other
+// warps 0). False when a wait gave up.
 template <int NK>
 __device__ bool exchange_sum (Word *slots, int grid, unsigned epoch, int &turn, bool ok, double (&v)[NK], double &out)
 {
@@ -163,59 +176,49 @@ __device__ bool exchange_sum (Word *slots, int grid, unsigned epoch, int &turn, 
     for (int k = 0; k < NK; k++)
       sh[k][w] = ws[k];
   __syncthreads ();
-  // kind by kind, so that a warp reads 512 consecutive bytes
-  Word *set = slots + (size_t) turn * kSlotKinds * grid * 2;
+  // [copy][kind][CTA], so that a warp reads 512 consecutive bytes
+  Word *set = slots + (size_t) turn * kSlotKinds * grid * 2 * kCopies;
   turn ^= 1;
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    if (w == k)
-      {
-        const double a = warp_sum (lane < nw ? sh[k][lane] : 0.0);
-        if (lane == 0)
-          put_value (set + ((size_t) k * grid + blockIdx.x) * 2, a, epoch);
-      }
-  double acc[NK];
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    acc[k] = 0.0;
-  for (int j = threadIdx.x; j < grid; j += blockDim.x)
+  double sum = 0.0;
+  if (w < NK)
     {
-      double got[NK];
-      ok = wait_for ([&] () {
-             bool all = true;
+      const double a = warp_sum (lane < nw ? sh[w][lane] : 0.0);
+      if (lane < kCopies)
+        put_value (set + (((size_t) lane * kSlotKinds + w) * grid + blockIdx.x) * 2, a, epoch);
+      const Word *mine = set + ((size_t) (blockIdx.x % kCopies) * kSlotKinds + w) * grid * 2;
+      constexpr int M = 5; // loads in flight: 160 CTAs
+      for (int j0 = 0; j0 < grid; j0 += 32 * M)
+        {
+          double got[M];
+          bool have[M];
 #pragma unroll
-             for (int k = 0; k < NK; k++)
-               {
-                 Word lo, hi;
-                 ld_words (set + ((size_t) k * grid + j) * 2, lo, hi);
-                 got[k] = value_of (lo, hi);
-                 all = all && tagged (lo, epoch) && tagged (hi, epoch);
-               }
-             return all;
-           })
-           && ok;
+          for (int m = 0; m < M; m++)
+            {
+              got[m] = 0.0;
+              have[m] = j0 + m * 32 + lane >= grid;
+            }
+          ok = wait_for ([&] () {
+                 bool all = true;
 #pragma unroll
-      for (int k = 0; k < NK; k++)
-        acc[k] = j < (int) blockDim.x ? got[k] : acc[k] + got[k];
+                 for (int m = 0; m < M; m++)
+                   if (!have[m])
+                     {
+                       Word lo, hi;
+                       ld_words (mine + (size_t) (j0 + m * 32 + lane) * 2, lo, hi);
+                       got[m] = value_of (lo, hi);
+                       have[m] = tagged (lo, epoch) && tagged (hi, epoch);
+                       all = all && have[m];
+                     }
+                 return all;
+               })
+               && ok;
+          __syncwarp ();
+          const double part = warp_sum_of<M> (got);
+          sum = j0 == 0 ? part : sum + part;
+        }
     }
-  const int used = (min (grid, (int) blockDim.x) + 31) / 32; // warps that read a slot
-  __syncthreads (); // sh has been read
-  if (w < used)
-    {
-      warp_sums<NK> (acc, ws);
-      if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NK; k++)
-          sh[k][w] = ws[k];
-    }
-  if (__syncthreads_or (!ok))
-    return false;
-  out = 0.0;
-#pragma unroll
-  for (int k = 0; k < NK; k++)
-    if (w == k)
-      out = warp_sum (lane < used ? sh[k][lane] : 0.0);
-  return true;
+  out = sum;
+  return __syncthreads_or (!ok) == 0;
 }
 
 // B consecutive values of the sliced matrix, staged (SM) or in global memory.

@@ -87,7 +87,7 @@ struct ResidentPlan
   bool matrix = false; // the CTA's part of the sliced matrix is staged in shared memory
   int o_vals = 0, o_cols = 0; // byte offsets of that copy
   int smem = 0;
-  unsigned long long *slots = nullptr; // words of the sums: [2][kSlotKinds][grid][2]
+  unsigned long long *slots = nullptr; // words of the sums: [2][kCopies][kSlotKinds][grid][2]
   // With the matrix in shared memory, p (q, g) and s (z) are published as
   // tagged words; else in place, a flag per CTA behind them, and a CTA waits
   // for the flags of CTAs need.x to need.y, whose rows its columns belong to.

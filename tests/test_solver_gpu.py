@@ -587,6 +587,25 @@ def test_auto_mode_on_systems_that_fit_the_sms(lib, cuda, grid, precision, preco
     A.close()
 
 
+@pytest.mark.parametrize("power", [0, -480, 480])
+@pytest.mark.parametrize("grid", [(40, 30), (200, 50)])
+def test_auto_mode_at_the_ends_of_the_exponents(lib, orc, cuda, grid, power):
+    """Right-hand sides of about 2**power: the grid's dot products leave the
+    exponents that are summed as integers. 1e-6 is asked for; the residual is
+    taken from the solution scaled back (exact, but for subnormals)."""
+    import torch
+    rp, c, v = shifted_q4(*grid)
+    n = 2 * grid[0] * grid[1]
+    A = bm.Matrix.from_bcsr(rp, c, v, 2)
+    b = np.random.default_rng(3).uniform(-1, 1, n)
+    x = torch.empty(n, dtype=torch.float64, device="cuda")
+    info = bm.Solver(A, "fp64", tol=1e-6).solve(dev(np.ldexp(b, power)), x)
+    assert info["status"] == bm.SUCCESS, info
+    y = np.ldexp(x.cpu().numpy(), -power)
+    assert np.linalg.norm(b - orc.bcsr_spmv(rp, c, v, 2, y)) <= 2e-6 * np.linalg.norm(b)
+    A.close()
+
+
 def test_auto_mode_solves_on_separate_streams(lib, cuda):
     """Four auto solves at once from four threads on four streams, staged and
     unstaged: each has the bits of the same solve run alone."""
