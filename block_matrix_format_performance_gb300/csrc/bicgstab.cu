@@ -101,6 +101,7 @@ template <typename T> struct Args
   // Sliced copy of a CSR or bs = 2 matrix (SellOp), or null.
   const int *soff, *scols;
   const T *svals;
+  bool stream; // the sliced copy does not stay in L2
   int nslices;
 };
 
@@ -229,6 +230,7 @@ constexpr int kSlice = 32;
 // steps' x in flight and the next three steps' values and columns behind
 // them: the walk is bound by latency otherwise. Rows are padded to the
 // slice's longest with zero blocks on a column the row already reads.
+// A copy larger than L2 is read evict-first, columns included (Stream).
 // 2000x500 Q4 grid, FP64, phases 2 and 4 by block rows and by slices: 84.5 and
 // 88.4 us -> 72.8 and 81.1 us (FP64 pipe 74 % -> 82 % busy, its work alone 61
 // and 64 us).
@@ -240,7 +242,7 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
     T v[B];
     int c;
   };
-  __device__ static __forceinline__ Step load (const T *v, const int *c, int k)
+  template <bool Stream> __device__ static __forceinline__ Step load (const T *v, const int *c, int k)
   {
     Step s;
     if constexpr (B == 1)
@@ -253,11 +255,13 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
       }
     else
       {
-        const float2 t = __ldg (reinterpret_cast<const float2 *> (v) + (size_t) k * kSlice);
+        const float2 *q = reinterpret_cast<const float2 *> (v) + (size_t) k * kSlice;
+        const float2 t = Stream ? __ldcs (q) : __ldg (q);
         s.v[0] = t.x;
         s.v[1] = t.y;
       }
-    s.c = __ldg (c + (size_t) k * (kSlice / B));
+    const int *q = c + (size_t) k * (kSlice / B);
+    s.c = Stream ? __ldcs (q) : __ldg (q);
     return s;
   }
   __device__ static __forceinline__ void gather (const T *x, int c, T (&xv)[B])
@@ -275,7 +279,18 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
     return acc;
   }
   template <class Epi>
-  __device__ static void run (const Args<T> &a, const T *x, T *y, Epi &e)
+  __device__ static __forceinline__ void run (const Args<T> &a, const T *x, T *y, Epi &e)
+  {
+    if constexpr (B == 1 || sizeof (T) == 4)
+      if (a.stream)
+        {
+          walk<true> (a, x, y, e);
+          return;
+        }
+    walk<false> (a, x, y, e);
+  }
+  template <bool Stream, class Epi>
+  __device__ static __forceinline__ void walk (const Args<T> &a, const T *x, T *y, Epi &e)
   {
     const int lane = threadIdx.x & 31;
     const int nw = (int) (gridDim.x * blockDim.x / kSlice);
@@ -305,7 +320,7 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
             Step s[U];
 #pragma unroll
             for (int u = 0; u < U; u++)
-              s[u] = load (v, c, u);
+              s[u] = load<Stream> (v, c, u);
             for (; k + 2 * U <= n; k += U)
               {
                 Step t[U];
@@ -315,7 +330,7 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
                   gather (x, s[u].c, xv[u]);
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                  t[u] = load (v, c, k + U + u);
+                  t[u] = load<Stream> (v, c, k + U + u);
 #pragma unroll
                 for (int u = 0; u < U; u++)
                   acc = add (s[u], xv[u], acc);
@@ -334,7 +349,7 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
           }
         for (; k < n; k++)
           {
-            const Step s = load (v, c, k);
+            const Step s = load<Stream> (v, c, k);
             T xv[B];
             gather (x, s.c, xv);
             acc = add (s, xv, acc);
@@ -1438,6 +1453,7 @@ Args<T> make_args (const bmfp_matrix_s *A, int64_t n, void *x, void *r, void *rh
   a.st = st;
   a.soff = a.scols = nullptr;
   a.svals = nullptr;
+  a.stream = false;
   a.nslices = 0;
   return a;
 }
@@ -1681,6 +1697,21 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
 // padding stays below an eighth (a structured grid's below 1 %) and it takes at
 // most a quarter of the free memory; the products walk the block rows
 // otherwise.
+// Whether the sliced copy's loads leave L2 to the vectors, by its bytes (L2
+// holds 129 MB). Where the copy mostly fits, reading it as usual keeps it there.
+// us per iteration as graphs / persistent, usual -> evicted first, Q4 operator:
+// FP32 blocks 86 MB 64 / 57 -> 64 / 59, 108 MB 86 / 80 -> 72 / 66, 180 MB
+// 124 / 111 -> 108 / 95 (43 MB 40 / 35 -> 45 / 43);
+// CSR FP32 137 MB 67 / 71 -> 71 / 73, 173 MB 93 / 101 -> 82 / 87; FP64 108 MB
+// 67 / 69 -> 68 / 73, 205 MB 117 / 119 -> 108 / 113, 432 MB 213 / 222 -> 202 / 213.
+// FP64 blocks, bound by the FP64 pipe, do not care: 216 MB 130 / 134 -> 132 / 135.
+bool streams (int dtype, int b, size_t bytes)
+{
+  if (b == 2)
+    return dtype == BMFP_R32F && bytes > (size_t) 96 << 20;
+  return bytes > (size_t) 160 << 20;
+}
+
 int WideEngine::build_sliced (cudaStream_t s)
 {
   const int nbr = A_->n_rows;
@@ -1736,6 +1767,7 @@ int WideEngine::build_sliced (cudaStream_t s)
   if (!svals_)
     return BMFP_SUCCESS;
   nslices_ = ns;
+  stream_ = streams (dtype_, B, o_off);
   spmv_kind_ = B == 2 ? kSell2 : kSell1;
   return BMFP_SUCCESS;
 }
@@ -1813,6 +1845,7 @@ template <typename T> struct WideEngine::ArgsOf
     a.soff = e.soff_;
     a.scols = e.scols_;
     a.svals = (const T *) e.svals_;
+    a.stream = e.stream_;
     a.nslices = e.nslices_;
     return a;
   }

@@ -191,6 +191,7 @@ private:
   void *svals_ = nullptr; // sliced copy of a bs = 2 matrix (one allocation), or null
   int *soff_ = nullptr, *scols_ = nullptr;
   int nslices_ = 0;
+  bool stream_ = false; // that copy is too large to stay in L2
   double *part_ = nullptr;
   size_t part_bytes_ = 0;
   DevState *state_ = nullptr;
