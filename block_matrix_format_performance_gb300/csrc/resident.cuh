@@ -29,10 +29,12 @@
 // everyone that its words have been read.
 //
 // us per iteration on the Q4 operator, as graphs and here: FP64 2 048 rows
-// 21.9 / 14.0, 20 000 21.5 / 17-21, 80 000 29.3 / 27.8, 500 000 66.6 / 64.2;
-// FP32 2 048 rows 19.8 / 12.6, 80 000 23.0 / 20.2, 180 000 31.4 / 22.9,
-// 500 000 39.8 / 34. Whole solves (K + 0.01 I): 200x50 FP64 4.38 -> 2.73 ms,
-// 1000x250 mixed 9.06 -> 5.07 ms.
+// 18 / 13, 20 000 22 / 15, 80 000 28 / 23, 180 000 39 / 32, 500 000 66 / 57;
+// FP32 2 048 rows 17 / 11, 20 000 20 / 13.5, 80 000 23 / 16.5, 180 000
+// 31 / 22, 500 000 41 / 26.5. Whole solves (K + 0.01 I): 200x50 FP64
+// 4.38 -> 2.73 ms, 1000x250 mixed 9.06 -> 5.07 ms. Of an iteration's 30 000
+// cycles at 20 000 rows the three sums take 17 000, the products 6 600, the
+// scalars 4 400.
 #pragma once
 
 // Threads per CTA at most: products from global memory live on the loads in
