@@ -1775,6 +1775,8 @@ int WideEngine::build_sliced (cudaStream_t s)
 // The resident iteration kernel's plan, for the auto launch mode: a sliced
 // matrix, no preconditioner or point Jacobi, fewer rows than the persistent
 // kernel's, and vectors that fit the SMs' shared memory beside each other.
+constexpr int kStagedRows = 1408;
+
 int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
 {
   const int B = spmv_kind_ == kSell2 ? 2 : 1;
@@ -1805,10 +1807,12 @@ int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
   BMFP_CUDA (cudaStreamSynchronize (s));
   const int64_t vals = (int64_t) steps.x * kSlice * B * S, cols = (int64_t) steps.x * (kSlice / B) * 4;
   P.o_vals = (int) ((vectors + 15) / 16 * 16);
-  // Staged and with tagged words up to 640 rows a CTA (97 000 in all): there
-  // the waits count (us per FP64 iteration at 80 000 rows 27.8, 29.3 as
-  // graphs); above, the tags' traffic does (180 000 rows 41.5 against 37.8).
-  P.matrix = P.rows <= 640 && P.o_vals + vals + cols <= most;
+  // Staged, and with tagged words, wherever it fits, up to the rows per CTA that
+  // were measured (us per iteration on the Q4 operator, staged against not:
+  // FP64 132 rows a CTA 14.9 / 16.2, 527 23.1 / 24.4, 697 24.0 / 25.6, 890
+  // 25.7 / 28.2, 1032 30.6 / 31.1; FP32 527 16.3 / 18.0, 890 17-19 / 20, 1185
+  // 19-21 / 21.9, 1382 20.9 / 22). From there on the tags' traffic grows.
+  P.matrix = P.rows <= kStagedRows && P.o_vals + vals + cols <= most;
   P.threads = std::min (P.rows, resident_threads ((int) S, P.matrix));
   P.o_cols = P.matrix ? (int) (P.o_vals + vals) : 0;
   P.smem = (int) (P.matrix ? P.o_vals + vals + cols : vectors);

@@ -31,7 +31,7 @@
 // us per iteration on the Q4 operator, as graphs and here: FP64 2 048 rows
 // 18 / 13, 20 000 22 / 15, 80 000 28 / 23, 180 000 39 / 32, 500 000 66 / 57;
 // FP32 2 048 rows 17 / 11, 20 000 20 / 13.5, 80 000 23 / 16.5, 180 000
-// 31 / 22, 500 000 41 / 26.5. Whole solves (K + 0.01 I): 200x50 FP64
+// 31 / 20, 500 000 41 / 26.5. Whole solves (K + 0.01 I): 200x50 FP64
 // 4.38 -> 2.73 ms, 1000x250 mixed 9.06 -> 5.07 ms. Of an iteration's 30 000
 // cycles at 20 000 rows the three sums take 17 000, the products 6 600, the
 // scalars 4 400.

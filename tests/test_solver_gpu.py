@@ -559,7 +559,7 @@ def shifted_q4(nx, ny, shift=0.02):
 def test_auto_mode_on_systems_that_fit_the_sms(lib, cuda, grid, precision, precond, fmt):
     """The auto launch mode's kernel for systems whose vectors fit the SMs'
     shared memory, from one partly filled CTA over the staged matrix's limit
-    (640 rows a CTA) to several thousand rows a CTA: the graph's answer, and
+    (1408 rows a CTA) to several thousand rows a CTA: the graph's answer, and
     the same bits every time."""
     import torch
     rp, c, v = shifted_q4(*grid)
@@ -640,7 +640,7 @@ def test_auto_mode_solves_on_separate_streams(lib, cuda):
     import threading
     import torch
     work = []
-    for grid in ((40, 30), (150, 65), (251, 250), (400, 150)):
+    for grid in ((40, 30), (150, 65), (251, 250), (600, 200)):
         rp, c, v = shifted_q4(*grid)
         A = bm.Matrix.from_bcsr(rp, c, v, 2)
         b = dev(np.random.default_rng(grid[0]).uniform(-1, 1, 2 * grid[0] * grid[1]))
