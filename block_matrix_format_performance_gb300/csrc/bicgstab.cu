@@ -1823,6 +1823,7 @@ int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
       resident_pub_bytes_ = 2 * vec;
       BMFP_CUDA (cudaMalloc (&resident_pub_, resident_pub_bytes_));
       BMFP_CUDA (cudaMemsetAsync (resident_pub_, 0, resident_pub_bytes_, s));
+      BMFP_CUDA (cudaStreamSynchronize (s)); // a solve on another stream would meet it
       P.pub[0] = (unsigned long long *) resident_pub_;
       P.pub[1] = (unsigned long long *) ((char *) resident_pub_ + vec);
     }

@@ -671,6 +671,41 @@ def test_auto_mode_solves_on_separate_streams(lib, cuda):
         assert torch.equal(x.view(torch.int64), work[k][2].view(torch.int64))
 
 
+def test_solver_created_on_a_busy_stream_solves_on_another(lib, cuda):
+    """Another thread keeps the creating stream busy, so that whatever creation
+    left on it would run into the solve on the second stream."""
+    import threading
+    import torch
+    rp, c, v = shifted_q4(200, 50)
+    A = bm.Matrix.from_bcsr(rp, c, v, 2)
+    b = dev(np.random.default_rng(1).uniform(-1, 1, 20000))
+    x0 = torch.empty_like(b)
+    bm.Solver(A, "fp64", tol=1e-12).solve(b, x0)
+    torch.cuda.synchronize()
+    made, other = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(3):
+        done = threading.Event()
+
+        def busy():
+            while not done.is_set():
+                with torch.cuda.stream(made):
+                    torch.cuda._sleep(2_000_000)  # about a millisecond; at most two of them queued
+                    e = torch.cuda.Event()
+                    torch.cuda._sleep(2_000_000)
+                    e.record(made)
+                e.synchronize()
+
+        t = threading.Thread(target=busy)
+        t.start()
+        s = bm.Solver(A, "fp64", tol=1e-12, stream=made.cuda_stream)
+        done.set()
+        x = torch.empty_like(b)
+        info = s.solve(b, x, stream=other.cuda_stream)
+        t.join()
+        assert info["status"] == bm.SUCCESS, info
+        assert torch.equal(x.view(torch.int64), x0.view(torch.int64))
+
+
 def test_concurrent_persistent_solves_on_separate_streams(lib, cuda):
     """Three persistent solves of a 1 000 000-row system launched at once from
     three host threads on three streams: cooperative launches that cannot be
