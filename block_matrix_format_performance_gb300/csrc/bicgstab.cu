@@ -2136,16 +2136,43 @@ int WideEngine::true_residual (const void *d_b, void *d_r, double *rr, double *b
 // WideEngine, without graphs, and without residual replacement (the
 // reference's plain recurrences).
 
-int barrier_selftest (double limit_s, int *fault, double *elapsed_s, cudaStream_t s)
+namespace
+{
+// One cooperative launch of a self-test kernel, a CTA per SM.
+cudaError_t launch_selftest (const void *fn, void **args, int sms, cudaStream_t s)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3 ((unsigned) sms);
+  cfg.blockDim = dim3 (kThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC (&cfg, fn, args);
+}
+
+int selftest_limits (double limit_s, int *sms)
 {
   if (!(limit_s > 0.0 && limit_s <= 1.0))
     return fail (BMFP_ERROR_INVALID_VALUE, "the self-test waits between 0 and 1 s (got %g)", limit_s);
-  int dev = 0, sms = 0, coop = 0;
+  int dev = 0, coop = 0;
   BMFP_CUDA (cudaGetDevice (&dev));
-  BMFP_CUDA (cudaDeviceGetAttribute (&sms, cudaDevAttrMultiProcessorCount, dev));
+  BMFP_CUDA (cudaDeviceGetAttribute (sms, cudaDevAttrMultiProcessorCount, dev));
   BMFP_CUDA (cudaDeviceGetAttribute (&coop, cudaDevAttrCooperativeLaunch, dev));
   if (!coop)
     return fail (BMFP_ERROR_NOT_SUPPORTED, "no cooperative launch on this device");
+  return BMFP_SUCCESS;
+}
+} // namespace
+
+int barrier_selftest (double limit_s, int *fault, double *elapsed_s, cudaStream_t s)
+{
+  int sms = 0;
+  const int rc = selftest_limits (limit_s, &sms);
+  if (rc != BMFP_SUCCESS)
+    return rc;
   DevState *st = nullptr;
   BMFP_CUDA (cudaMalloc (&st, sizeof (DevState)));
   cudaEvent_t a = nullptr, b = nullptr;
@@ -2160,16 +2187,7 @@ int barrier_selftest (double limit_s, int *fault, double *elapsed_s, cudaStream_
     {
       unsigned long long limit_ns = (unsigned long long) (limit_s * 1e9);
       void *args[] = { &st, &limit_ns };
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3 ((unsigned) sms);
-      cfg.blockDim = dim3 (kThreads);
-      cfg.stream = s;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeCooperative;
-      attr[0].val.cooperative = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      e = cudaLaunchKernelExC (&cfg, (const void *) barrier_selftest_kernel, args);
+      e = launch_selftest ((const void *) barrier_selftest_kernel, args, sms, s);
     }
   DevState h{};
   if (e == cudaSuccess)
@@ -2192,6 +2210,45 @@ int barrier_selftest (double limit_s, int *fault, double *elapsed_s, cudaStream_
     *fault = h.fault;
   if (elapsed_s)
     *elapsed_s = ms * 1e-3;
+  return BMFP_SUCCESS;
+}
+
+int resident_selftest (double limit_s, int *faults, cudaStream_t s)
+{
+  int sms = 0;
+  const int rc = selftest_limits (limit_s, &sms);
+  if (rc != BMFP_SUCCESS)
+    return rc;
+  const size_t words = sizeof (Word) * 2 * kSlotKinds * 2 * kCopies * (size_t) (sms + 1);
+  const size_t flags = sizeof (unsigned) * kFlagStride * (size_t) (sms + 1);
+  char *mem = nullptr;
+  BMFP_CUDA (cudaMalloc (&mem, words + flags + sizeof (DevState)));
+  DevState *st = (DevState *) (mem + words + flags);
+  cudaError_t e = cudaSuccess;
+  int bits = 0;
+  for (int which = 0; which < 3 && e == cudaSuccess; which++)
+    {
+      e = cudaMemsetAsync (mem, 0, words + flags + sizeof (DevState), s);
+      unsigned long long limit_ns = (unsigned long long) (limit_s * 1e9);
+      Word *slots = (Word *) mem;
+      unsigned *f = (unsigned *) (mem + words);
+      void *args[] = { &st, &slots, &f, &which, &limit_ns };
+      if (e == cudaSuccess)
+        e = launch_selftest ((const void *) resident_selftest_kernel, args, sms, s);
+      DevState h{};
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync (&h, st, sizeof (DevState), cudaMemcpyDeviceToHost, s);
+      if (e == cudaSuccess)
+        e = cudaStreamSynchronize (s);
+      // the first CTA's write-back counts only if it did come after the fault
+      if (e == cudaSuccess && h.fault && (which != 2 || h.gen == 1))
+        bits |= 1 << which;
+    }
+  cudaFree (mem);
+  if (e != cudaSuccess)
+    return cuda_fail (e, "self-test of the resident kernel's waits", __FILE__, __LINE__);
+  if (faults)
+    *faults = bits;
   return BMFP_SUCCESS;
 }
 

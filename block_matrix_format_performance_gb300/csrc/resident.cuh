@@ -131,8 +131,9 @@ __device__ __forceinline__ bool get_flag (const unsigned *f, unsigned epoch)
   return (int) (v - epoch) >= 0;
 }
 
-// Looks until `ready`, for at most kBarrierLimitNs; false when it gave up.
-template <class F> __device__ __forceinline__ bool wait_for (F ready)
+// Looks until `ready`, for at most limit_ns; false when it gave up.
+template <class F>
+__device__ __forceinline__ bool wait_for (F ready, unsigned long long limit_ns = kBarrierLimitNs)
 {
   if (ready ())
     return true;
@@ -143,7 +144,7 @@ template <class F> __device__ __forceinline__ bool wait_for (F ready)
         const unsigned long long now = global_ns ();
         if (t0 == 0)
           t0 = now;
-        else if (now - t0 > kBarrierLimitNs)
+        else if (now - t0 > limit_ns)
           return false;
       }
   return true;
@@ -151,14 +152,15 @@ template <class F> __device__ __forceinline__ bool wait_for (F ready)
 
 // This CTA's part of a vector is stored (in place): releases its flag and
 // waits for the parts its rows read. False when a wait gave up.
-__device__ __forceinline__ bool publish (unsigned *flags, int2 need, unsigned epoch)
+__device__ __forceinline__ bool publish (unsigned *flags, int2 need, unsigned epoch,
+                                         unsigned long long limit_ns = kBarrierLimitNs)
 {
   __syncthreads ();
   if (threadIdx.x == 0)
     put_flag (flags + blockIdx.x * kFlagStride, epoch);
   bool ok = true;
   for (int j = need.x + (int) threadIdx.x; j <= need.y; j += blockDim.x)
-    ok = wait_for ([&] () { return get_flag (flags + j * kFlagStride, epoch); }) && ok;
+    ok = wait_for ([&] () { return get_flag (flags + j * kFlagStride, epoch); }, limit_ns) && ok;
   return __syncthreads_or (!ok) == 0;
 }
 
@@ -167,7 +169,8 @@ __device__ __forceinline__ bool publish (unsigned *flags, int2 need, unsigned ep
 // (k < NK <= 4 <= the CTA's warps) returns kind k's sum on every lane (other
 // warps 0). False when a wait gave up.
 template <int NK>
-__device__ bool exchange_sum (Word *slots, int grid, unsigned epoch, int &turn, bool ok, double (&v)[NK], double &out)
+__device__ bool exchange_sum (Word *slots, int grid, unsigned epoch, int &turn, bool ok, double (&v)[NK], double &out,
+                              unsigned long long limit_ns = kBarrierLimitNs)
 {
   __shared__ double sh[NK][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -212,7 +215,7 @@ __device__ bool exchange_sum (Word *slots, int grid, unsigned epoch, int &turn, 
                        all = all && have[m];
                      }
                  return all;
-               })
+               }, limit_ns)
                && ok;
           __syncwarp ();
           const double part = warp_sum_of<M> (got);
@@ -406,6 +409,22 @@ __device__ __forceinline__ void resident_decide (DevState *S, double sum, bool r
   __syncthreads ();
 }
 
+// A wait gave up. Only the host clears the word: a CTA that ends its launch
+// well may do so after this one (store_state).
+__device__ __forceinline__ void record_fault (DevState *st)
+{
+  cuda::atomic_ref<int, cuda::thread_scope_device> (st->fault).store (1, cuda::memory_order_relaxed);
+}
+
+// The state at the end of a launch, by one thread: all but the fault word.
+__device__ __forceinline__ void store_state (DevState *st, const DevState &S)
+{
+  static_assert (offsetof (DevState, pad) == offsetof (DevState, fault) + 4
+                   && sizeof (DevState) == offsetof (DevState, fault) + 8,
+                 "nothing but padding behind the fault word");
+  memcpy (st, &S, offsetof (DevState, fault));
+}
+
 template <typename T, int B, int PK, bool SM>
 __global__ void __launch_bounds__ (resident_threads (sizeof (T), SM), 1) resident_kernel (Args<T> a, ResidentPlan P, int iters)
 {
@@ -419,8 +438,8 @@ __global__ void __launch_bounds__ (resident_threads (sizeof (T), SM), 1) residen
   if (t == 0)
     S = *a.st;
   __syncthreads ();
-  if (S.done)
-    return; // every CTA reads the same word: it was written before this launch
+  if (S.done || S.fault)
+    return; // every CTA reads the same words: they were written before this launch
   unsigned epoch = S.gen; // number of the last exchange
   int turn = 0;          // set of the next sum's words
   const int grid = P.grid;
@@ -604,7 +623,7 @@ __global__ void __launch_bounds__ (resident_threads (sizeof (T), SM), 1) residen
   if (!ok)
     {
       if (t == 0)
-        cuda::atomic_ref<int, cuda::thread_scope_device> (a.st->fault).store (1, cuda::memory_order_relaxed);
+        record_fault (a.st);
       return;
     }
   __syncthreads ();
@@ -619,8 +638,7 @@ __global__ void __launch_bounds__ (resident_threads (sizeof (T), SM), 1) residen
     {
       S.gen = epoch;
       S.arrive = 0;
-      S.fault = 0;
-      *a.st = S;
+      store_state (a.st, S);
     }
 }
 
@@ -654,4 +672,39 @@ __global__ void resident_need_kernel (int64_t n, int rows, int b, const int *sof
       need[self].y = lo == INT_MAX ? self : (int) (((int64_t) hi * b + b - 1) / rows);
       atomicMax (&need[gridDim.x].x, s1 - s0);
     }
+}
+
+// The waits above run out on purpose, which = 0: a sum over one CTA more than
+// the grid holds; 1: a flag that nothing releases; 2: the same in all CTAs but
+// the first, which ends its launch after one of them has recorded its fault.
+__global__ void resident_selftest_kernel (DevState *st, Word *slots, unsigned *flags, int which,
+                                          unsigned long long limit_ns)
+{
+  __shared__ DevState S;
+  const int grid = (int) gridDim.x;
+  if (threadIdx.x == 0)
+    S = *st;
+  __syncthreads ();
+  bool ok;
+  if (which == 0)
+    {
+      int turn = 0;
+      double in[3] = { 1.0, 1.0, 1.0 }, sum;
+      ok = exchange_sum<3> (slots, grid + 1, 1, turn, true, in, sum, limit_ns);
+    }
+  else if (which == 1 || blockIdx.x > 0)
+    ok = publish (flags, make_int2 (0, grid), 1, limit_ns);
+  else
+    {
+      if (threadIdx.x == 0)
+        {
+          cuda::atomic_ref<int, cuda::thread_scope_device> fault (st->fault);
+          wait_for ([&] () { return fault.load (cuda::memory_order_relaxed) != 0; }, 4 * limit_ns);
+          S.gen = 1;
+          store_state (st, S);
+        }
+      return;
+    }
+  if (!ok && threadIdx.x == 0)
+    record_fault (st);
 }

@@ -56,7 +56,7 @@ struct DevState
   int replacements;
   unsigned arrive; // CTAs of the running kernel that have written their partials
   unsigned gen;    // grid barriers passed by the persistent iteration kernel
-  int fault;       // a grid barrier of that kernel gave up waiting
+  int fault;       // a wait of that kernel (or the resident one) gave up; only the host clears it
   int pad;
 };
 
@@ -230,6 +230,7 @@ int raw_solve_grid (int64_t n, int *grid);
 // for one CTA more than the grid holds) after limit_s: reports the fault flag
 // the timed-out CTAs set and how long the launch took.
 int barrier_selftest (double limit_s, int *fault, double *elapsed_s, cudaStream_t s);
+int resident_selftest (double limit_s, int *faults, cudaStream_t s);
 int raw_jacobi (const RawSolve &b, cudaStream_t stream);
 int raw_start (const RawSolve &b, const void *d_rhs, double tol, int max_iter, cudaStream_t stream);
 int raw_phase (const RawSolve &b, int phase, cudaStream_t stream);

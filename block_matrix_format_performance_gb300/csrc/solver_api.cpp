@@ -510,6 +510,11 @@ int bmfp_selftest_barrier_timeout (double limit_seconds, int *fault, double *ela
   return bmfp::barrier_selftest (limit_seconds, fault, elapsed_seconds, as_stream (stream));
 }
 
+int bmfp_selftest_resident_timeout (double limit_seconds, int *faults, void *stream)
+{
+  return bmfp::resident_selftest (limit_seconds, faults, as_stream (stream));
+}
+
 } // extern "C"
 
 struct bmfp_batch_s

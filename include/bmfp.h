@@ -373,6 +373,11 @@ BMFP_API int bmfp_solver_destroy (bmfp_solver_t s);
  * stays usable. Synchronises the stream. */
 BMFP_API int bmfp_selftest_barrier_timeout (double limit_seconds, int *fault, double *elapsed_seconds,
                                             void *stream);
+/* The same for the auto mode's shared-memory kernel, three launches whose waits
+ * run out after limit_seconds: the grid's sums (bit 0 of *faults when the flag
+ * was recorded), its flags (bit 1), and its flags while one CTA ends the launch
+ * well after the others' fault, which must stay recorded (bit 2). 7 is expected. */
+BMFP_API int bmfp_selftest_resident_timeout (double limit_seconds, int *faults, void *stream);
 
 /* -------------------------------------------------------------- batched ---
  * Many independent square systems of uneven size solved by ONE persistent

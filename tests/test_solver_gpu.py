@@ -521,6 +521,22 @@ def test_grid_barrier_wait_runs_out_and_reports(lib, cuda):
     assert info["status"] == bm.SUCCESS
 
 
+def test_resident_kernel_waits_run_out_and_report(lib, cuda):
+    """The same for the kernel of the auto mode below a million rows: its sums
+    and its flags give up and record it, and a CTA that ends its launch well
+    afterwards leaves the record (a timeout that it wiped would let the run go on
+    from vectors of two iterations). The next solve is right."""
+    import ctypes
+    faults = ctypes.c_int(0)
+    assert lib.bmfp_selftest_resident_timeout(0.02, ctypes.byref(faults), None) == bm.SUCCESS, lib.bmfp_last_error()
+    assert faults.value == 7
+    assert lib.bmfp_selftest_resident_timeout(2.0, None, None) == bm.ERROR_INVALID_VALUE
+    rp, c, v, b = bm.gen_q4_elasticity(60, 15)
+    A = bm.Matrix.from_bcsr(rp, c, v, 2)
+    x, info = bm.Solver(A, "fp64").solve_host(b)
+    assert info["status"] == bm.SUCCESS
+
+
 def test_auto_launch_mode_takes_the_persistent_kernel_from_a_million_rows(lib, cuda):
     """A 1 000 000-row system under the auto launch mode runs the persistent
     kernel (its bits equal the explicit persistent launch's and, on the same
