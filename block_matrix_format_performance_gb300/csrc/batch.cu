@@ -151,7 +151,9 @@ struct TeamIdx
 };
 
 // Row-group loop of one SpMV over the team: FLAT (bs 2, 16-byte loads),
-// CSR (bs 1) or TPR (any bs <= 32, warp per block row).
+// CSR (bs 1) or TPR (any bs <= 32, warp per block row). The vector was written
+// by other CTAs of the same launch before a cluster barrier, so the products
+// load it coherently (XCoh).
 enum BatchOp
 {
   kOpFlat2 = 0,
@@ -170,7 +172,7 @@ template <typename T> struct TeamOp<T, kOpFlat2>
       pair_rows (S, ix, x, y, e);
     else
       for (int64_t row = ix.group0; row < S.nbr; row += ix.group_stride)
-        core::flat_row<T, 2, 2, 4> ((int) row, S.rp, S.cols, S.vals, x, y, e);
+        core::flat_row<T, 2, 2, 4, dev::XCoh> ((int) row, S.rp, S.cols, S.vals, x, y, e);
   }
   // FP32: two lanes share a block row, a whole block each per step, five steps
   // (ten blocks: a row of a Q4 grid) at once, the next row's offsets ahead. A
@@ -211,7 +213,7 @@ template <typename T> struct TeamOp<T, kOpFlat2>
               }
 #pragma unroll
             for (int u = 0; u < U; u++)
-              xv[u] = __ldg (reinterpret_cast<const float2 *> (x) + c[u]);
+              dev::XCoh::ld2 (x + (size_t) c[u] * 2, xv[u].x, xv[u].y);
 #pragma unroll
             for (int u = 0; u < U; u++)
               if (b0 + 2 * u < end)
@@ -242,7 +244,7 @@ template <typename T> struct TeamOp<T, kOpCsr>
   __device__ static void run (const TeamSys<T> &S, const TeamIdx &ix, const T *x, T *y, Epi &e)
   {
     for (int64_t row = ix.group0; row < S.nbr; row += ix.group_stride)
-      core::csr_row<T, 4> ((int) row, S.rp, S.cols, S.vals, x, y, e);
+      core::csr_row<T, 4, dev::XCoh> ((int) row, S.rp, S.cols, S.vals, x, y, e);
   }
 };
 template <typename T> struct TeamOp<T, kOpTpr>
@@ -252,7 +254,7 @@ template <typename T> struct TeamOp<T, kOpTpr>
   __device__ static void run (const TeamSys<T> &S, const TeamIdx &ix, const T *x, T *y, Epi &e)
   {
     for (int64_t row = ix.group0; row < S.nbr; row += ix.group_stride)
-      core::tpr_row<T, 0> ((int) row, S.bs, S.rp, S.cols, S.vals, x, y, e);
+      core::tpr_row<T, 0, dev::XCoh> ((int) row, S.bs, S.rp, S.cols, S.vals, x, y, e);
   }
 };
 
