@@ -422,7 +422,7 @@ __device__ __forceinline__ void store_state (DevState *st, const DevState &S)
   static_assert (offsetof (DevState, pad) == offsetof (DevState, fault) + 4
                    && sizeof (DevState) == offsetof (DevState, fault) + 8,
                  "nothing but padding behind the fault word");
-  memcpy (st, &S, offsetof (DevState, fault));
+  memcpy (__builtin_assume_aligned (st, 8), __builtin_assume_aligned (&S, 8), offsetof (DevState, fault));
 }
 
 template <typename T, int B, int PK, bool SM>
