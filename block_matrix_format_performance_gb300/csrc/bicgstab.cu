@@ -230,6 +230,11 @@ constexpr int kSlice = 32;
 // steps' x in flight and the next three steps' values and columns behind
 // them: the walk is bound by latency otherwise. Rows are padded to the
 // slice's longest with zero blocks on a column the row already reads.
+// Steps that fill no group run together too: taken one by one, each waited for its
+// column and then its x, and rows of 5 to 8 blocks were slower than the walk of
+// the block rows (us per iteration, block rows / one by one / together: FP32,
+// 1.2 M rows, persistent, 7 blocks 67 / 92 / 68; FP64, 400 000 rows, graphs with
+// one CTA per SM, 5 blocks 64 / 73 / 55, 8 blocks 81 / 92 / 76).
 // A copy larger than L2 is read evict-first, columns included (Stream).
 // 2000x500 Q4 grid, FP64, phases 2 and 4 by block rows and by slices: 84.5 and
 // 88.4 us -> 72.8 and 81.1 us (FP64 pipe 74 % -> 82 % busy, its work alone 61
@@ -237,6 +242,10 @@ constexpr int kSlice = 32;
 template <typename T, int B, class XL = dev::XNc> struct SellOp
 {
   static constexpr int U = sizeof (T) == 4 ? 9 : B == 1 ? 6 : 3;
+  // Steps that fill no group: in the FP64 phase kernels first, with the first
+  // group on its way behind them, else last (the persistent kernel's 80 registers
+  // do not hold both).
+  static constexpr bool kAhead = sizeof (T) == 8 && std::is_same_v<XL, dev::XNc>;
   struct Step
   {
     T v[B];
@@ -314,13 +323,31 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
         const int *c = a.scols + (size_t) beg * (kSlice / B) + lane / B;
         const int n = end - beg;
         T acc = 0;
-        int k = 0;
+        // The odd steps, together: past their end the last again, not added.
+        auto odd = [&] (int from, int left) {
+          Step t[U - 1];
+          T xv[U - 1][B];
+#pragma unroll
+          for (int u = 0; u < U - 1; u++)
+            t[u] = load<Stream> (v, c, from + min (u, left - 1));
+#pragma unroll
+          for (int u = 0; u < U - 1; u++)
+            gather (x, t[u].c, xv[u]);
+#pragma unroll
+          for (int u = 0; u < U - 1; u++)
+            if (u < left)
+              acc = add (t[u], xv[u], acc);
+        };
+        int k = kAhead ? n % U : 0;
+        Step s[U];
+        if (n >= U)
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            s[u] = load<Stream> (v, c, k + u);
+        if (kAhead && k > 0)
+          odd (0, k);
         if (n >= U)
           {
-            Step s[U];
-#pragma unroll
-            for (int u = 0; u < U; u++)
-              s[u] = load<Stream> (v, c, u);
             for (; k + 2 * U <= n; k += U)
               {
                 Step t[U];
@@ -347,13 +374,8 @@ template <typename T, int B, class XL = dev::XNc> struct SellOp
               acc = add (s[u], xv[u], acc);
             k += U;
           }
-        for (; k < n; k++)
-          {
-            const Step s = load<Stream> (v, c, k);
-            T xv[B];
-            gather (x, s.c, xv);
-            acc = add (s, xv, acc);
-          }
+        if (!kAhead && k < n)
+          odd (k, n - k);
         if (i < a.n)
           {
             y[i] = acc;

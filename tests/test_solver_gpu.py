@@ -137,6 +137,61 @@ def test_sliced_copy_of_block_size_two(lib, cuda, nbr, spread, precision):
     A.close()
 
 
+def even_rows(nbr, k, b, dt=np.float64):
+    """nbr block rows of k blocks of size b each, a dominant diagonal."""
+    rng = np.random.default_rng(k)
+    c = np.sort((np.arange(nbr)[:, None] + np.arange(k)[None, :] * 3) % nbr, axis=1).astype(np.int32)
+    v = rng.uniform(-1, 1, (nbr * k, b, b))
+    v[np.repeat(np.arange(nbr), k) == c.reshape(-1)] += 1.5 * b * k * np.eye(b)
+    return (np.arange(nbr + 1) * k).astype(np.int32), c.reshape(-1), v.reshape(-1).astype(dt)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("b", [1, 2])
+@pytest.mark.parametrize("k", [1, 2, 4, 5, 7, 8, 10, 13, 17, 19])
+def test_sliced_products_at_every_remainder(lib, cuda, k, b, precision):
+    """Rows that are no multiple of the steps the sliced product takes at once,
+    shorter than them and longer: graphs and the persistent kernel agree in every
+    bit and meet the residual asked for."""
+    dt = np.float64 if precision == "fp64" else np.float32
+    nbr = 1009
+    rp, c, v = even_rows(nbr, k, b, dt)
+    A = bm.Matrix.from_csr(rp, c, v, nbr) if b == 1 else bm.Matrix.from_bcsr(rp, c, v, b)
+    rhs = np.random.default_rng(k).uniform(-1, 1, nbr * b).astype(dt)
+    tol = 1e-10 if precision == "fp64" else 1e-5
+    out = []
+    for mode in ("graph", "persistent"):
+        x, info = bm.Solver(A, precision, tol=tol, ctas_per_sm=3, launch_mode=mode).solve_host(rhs)
+        assert info["status"] == bm.SUCCESS, info
+        out.append(x)
+    assert _same_bits(*out)
+    K = bcsr_dense_csr(rp, c, v, b)
+    assert np.linalg.norm(rhs - K @ out[0]) / np.linalg.norm(rhs) < 2 * tol
+    A.close()
+
+
+@pytest.mark.parametrize("short", [7])
+def test_sliced_products_of_short_rows_take_no_longer(lib, cuda, short):
+    """FP32, 1.2 million rows, persistent: seven blocks a row against nine. Odd
+    steps taken one by one made the shorter rows 1.35 times as slow."""
+    import torch
+    us = {}
+    for k in (short, 9):
+        rp, c, v = even_rows(600000, k, 2)
+        A = bm.Matrix.from_bcsr(rp, c, v, 2)
+        b = dev(np.random.default_rng(1).uniform(-1, 1, 1200000))
+        x = torch.empty_like(b)
+        t = []
+        for it in (20, 4):  # the dominant diagonal reaches FP32's floor after about 30 iterations
+            s = bm.Solver(A, "fp32", tol=1e-30, max_iters=it, check_true_residual=1, launch_mode="persistent")
+            t.append(min((i["seconds"], i["iterations"]) for i in (s.solve(b, x) for _ in range(10))))
+            s.close()
+        assert t[0][1] - t[1][1] >= 12, t
+        us[k] = (t[0][0] - t[1][0]) / (t[0][1] - t[1][1]) * 1e6
+        A.close()
+    assert us[short] < 1.15 * us[9], us
+
+
 def test_csr_matrix_solve_like_the_reference(lib, orc, cuda):
     """The reference solves CSR (csr_matrix_class); bs = 0 handles go through
     the CSR phase kernels."""
