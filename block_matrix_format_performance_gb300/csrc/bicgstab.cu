@@ -1714,26 +1714,30 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   return iterate_ ? BMFP_SUCCESS : capture (capture_stream_);
 }
 
+// Whether the sliced copy's loads leave L2 (129 MB) to the vectors. FP32 blocks: once
+// the copy and the eight vectors of an iteration no longer fit together, whatever
+// the row length. us per iteration as graphs, usual -> evicted first, by blocks a
+// row and MB of copy + vectors: 3 blocks 70 + 75 118 -> 104; 5 blocks 70 + 45
+// 81 -> 79, 84 + 54 100 -> 87; 7 blocks 70 + 32 62 -> 67, 84 + 38 80 -> 74; 8 blocks
+// 70 + 28 58 -> 65, 84 + 34 76 -> 73, 96 + 38 86 -> 77; 9 blocks 70 + 25 57 -> 64,
+// 84 + 30 70 -> 71, 96 + 34 82 -> 76, 140 + 50 110 -> 95; 13 blocks 84 + 21 65 -> 71,
+// 96 + 24 77 -> 76, 110 + 27 92 -> 83.
+// CSR, by the copy alone, as graphs / persistent: FP32 137 MB 67 / 71 -> 71 / 73, 173 MB
+// 93 / 101 -> 82 / 87; FP64 108 MB 67 / 69 -> 68 / 73, 205 MB 117 / 119 -> 108 / 113, 432 MB
+// 213 / 222 -> 202 / 213.
+// FP64 blocks, bound by the FP64 pipe, do not care: 216 MB 130 / 134 -> 132 / 135.
+bool streams (int dtype, int b, size_t bytes, int64_t n)
+{
+  if (b == 2)
+    return dtype == BMFP_R32F && bytes + 8 * sizeof (float) * (size_t) n > (size_t) 115 << 20;
+  return bytes > (size_t) 160 << 20;
+}
+
 // The sliced copy of a CSR or bs = 2 matrix: one more pass over it at creation and as
 // many bytes again, kept where rows of one slice differ so little that the
 // padding stays below an eighth (a structured grid's below 1 %) and it takes at
 // most a quarter of the free memory; the products walk the block rows
 // otherwise.
-// Whether the sliced copy's loads leave L2 to the vectors, by its bytes (L2
-// holds 129 MB). Where the copy mostly fits, reading it as usual keeps it there.
-// us per iteration as graphs / persistent, usual -> evicted first, Q4 operator:
-// FP32 blocks 86 MB 64 / 57 -> 64 / 59, 108 MB 86 / 80 -> 72 / 66, 180 MB
-// 124 / 111 -> 108 / 95 (43 MB 40 / 35 -> 45 / 43);
-// CSR FP32 137 MB 67 / 71 -> 71 / 73, 173 MB 93 / 101 -> 82 / 87; FP64 108 MB
-// 67 / 69 -> 68 / 73, 205 MB 117 / 119 -> 108 / 113, 432 MB 213 / 222 -> 202 / 213.
-// FP64 blocks, bound by the FP64 pipe, do not care: 216 MB 130 / 134 -> 132 / 135.
-bool streams (int dtype, int b, size_t bytes)
-{
-  if (b == 2)
-    return dtype == BMFP_R32F && bytes > (size_t) 96 << 20;
-  return bytes > (size_t) 160 << 20;
-}
-
 int WideEngine::build_sliced (cudaStream_t s)
 {
   const int nbr = A_->n_rows;
@@ -1789,7 +1793,7 @@ int WideEngine::build_sliced (cudaStream_t s)
   if (!svals_)
     return BMFP_SUCCESS;
   nslices_ = ns;
-  stream_ = streams (dtype_, B, o_off);
+  stream_ = streams (dtype_, B, o_off, n_);
   spmv_kind_ = B == 2 ? kSell2 : kSell1;
   return BMFP_SUCCESS;
 }
