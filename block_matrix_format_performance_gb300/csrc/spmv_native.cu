@@ -151,32 +151,50 @@ __global__ void __launch_bounds__ (kThreads)
 // G lanes per row, with G a fraction of the average row: a row's sum costs
 // log2 G warp-wide FP64 adds beside its multiply-adds, and GB300's FP64 pipe
 // charges each of them in full. A row far above the average would then run
-// long on its few lanes, so the warp takes such rows together afterwards.
+// long on its few lanes, so a whole warp takes it, and not one of its own CTA:
+// long rows that lie together (the last ones of a bordered system) would queue
+// there. CTA c looks at the eights of rows c, c + C, c + 2 C ... of the C CTAs, and
+// warp w takes the w-th row of each. us, by 32 lanes a row / by the warp of the
+// row's own group / this: 200 000 rows of 18, FP64, 8 rows of 100 000 entries at the
+// end 1641 / 11690 / 1545, 64 of 20 000 408 / 2510 / 337; the 1000x250 elasticity operator,
+// without long rows, 215 / 36.8 / 36.9. (A warp looking at rows W apart instead, no
+// barrier: 37.9, and rows of 5 in FP32 8.9 -> 11.9.)
 template <typename T, int G>
 __global__ void __launch_bounds__ (kThreads)
   csr_subwarp_kernel (int n_rows, const int *__restrict__ row_ptr, const int *__restrict__ cols,
                       const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
 {
   constexpr int kLongRow = 16 * G + 48;
+  constexpr int kWarps = kThreads / 32;
+  static_assert (kWarps == 8, "a warp to each row of an eight");
   const int64_t row = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / G;
   core::NoEpilogue epi;
-  bool wide = false;
-  if (row < n_rows)
-    {
-      wide = G < 32 && __ldg (row_ptr + row + 1) - __ldg (row_ptr + row) > kLongRow;
-      if (!wide)
-        core::csr_row<T, G> ((int) row, row_ptr, cols, vals, x, y, epi);
-    }
+  // the t-th row that this CTA looks at (past the last row: an empty one), its
+  // offsets on their way while the lanes' own rows run
+  auto row_at = [&] (int t) { return ((int64_t) (t / 8) * gridDim.x + blockIdx.x) * 8 + t % 8; };
+  auto offset = [&] (int64_t r) { return __ldg (row_ptr + min (r, (int64_t) n_rows)); };
+  int beg = 0, end = 0;
   if constexpr (G < 32)
     {
-      unsigned left = __ballot_sync (0xffffffffu, wide && (threadIdx.x & (G - 1)) == 0);
-      while (left)
-        {
-          const int src = __ffs (left) - 1;
-          left &= left - 1;
-          core::csr_row<T, 32> ((int) __shfl_sync (0xffffffffu, (int) row, src), row_ptr, cols, vals, x, y, epi);
-        }
+      beg = offset (row_at (threadIdx.x));
+      end = offset (row_at (threadIdx.x) + 1);
     }
+  if (row < n_rows && (G == 32 || offset (row + 1) - offset (row) <= kLongRow))
+    core::csr_row<T, G> ((int) row, row_ptr, cols, vals, x, y, epi);
+  const bool wide = end - beg > kLongRow;
+  if constexpr (G < 32)
+    if (__syncthreads_or (wide))
+      {
+        __shared__ unsigned masks[kWarps];
+        const int w = threadIdx.x >> 5;
+        const unsigned mask = __ballot_sync (0xffffffffu, wide);
+        if ((threadIdx.x & 31) == 0)
+          masks[w] = mask;
+        __syncthreads ();
+        for (int q = 0; q < kWarps; q++)
+          for (unsigned left = masks[q] & (0x01010101u << w); left; left &= left - 1)
+            core::csr_row<T, 32> ((int) row_at (q * 32 + __ffs (left) - 1), row_ptr, cols, vals, x, y, epi);
+      }
 }
 
 // ---------------------------------------------------------------- dispatch

@@ -197,6 +197,38 @@ def test_csr_rows_far_above_the_average(lib, orc, cuda, lanes, dtype):
     assert np.all(np.abs(y[:1003] - orc.csr_spmv(rp, c, v, x)) <= spmv_tolerance(orc, rp, c, v, x, dtype))
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("avg", [4, 18, 40])
+def test_csr_long_rows_that_lie_together(lib, orc, cuda, avg, dtype):
+    """The last eight rows far above the average, as in a bordered system: right,
+    and not much longer than one such row alone (one warp after the other took
+    them seven times as long)."""
+    import torch
+    rng = np.random.default_rng(avg)
+    n, times = 50000, {}
+    for many in (1, 8):
+        counts = rng.integers(avg - 2, avg + 3, n)
+        counts[n - many:] = 20000
+        rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+        c = rng.integers(0, n, rp[-1]).astype(np.int32)
+        v, x = rng.uniform(-1, 1, c.size).astype(dtype), rng.uniform(-1, 1, n).astype(dtype)
+        d = [dev(a) for a in (rp, c, v, x)]
+        d_y = torch.full((n + GUARD,), float("nan"), dtype=d[3].dtype, device="cuda")
+        t = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            bm.csr_spmv(bm.CSR_NATIVE, *d, d_y)
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+        times[many] = min(t)
+        y = d_y.cpu().numpy()
+        assert np.isnan(y[n:]).all()
+        assert np.all(np.abs(y[:n] - orc.csr_spmv(rp, c, v, x)) <= spmv_tolerance(orc, rp, c, v, x, dtype))
+    assert times[8] < 3 * times[1], times
+
+
 def tiled_bcsr(bs, dtype, seed, kind):
     """A BCSR matrix with enough blocks for the row-tile kernel. kind: rows of
     0-15 blocks; mostly empty rows; rows far longer than a tile among them."""
