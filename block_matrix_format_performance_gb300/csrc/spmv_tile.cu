@@ -109,19 +109,17 @@ constexpr int blocks_in_flight (int bs, int bytes)
   return bs <= 3 ? 3 : bs <= 6 ? 2 : bs <= 12 && bytes == 4 ? 2 : 1;
 }
 
+// One pass over nr rows from r0 on, n blocks from block B0 on, by the whole CTA.
 template <typename T, int BSC, int V, bool PAD>
-__global__ void __launch_bounds__ (kThreads, BSC == 3 ? 10 : 8)
-  tile_kernel (int nbr, int bs_rt, TilePlan P, const int *__restrict__ row_ptr, const int *__restrict__ cols,
-               const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
+__device__ __forceinline__ void tile_pass (int nbr, int bs_rt, const TilePlan &P, const int *__restrict__ row_ptr,
+                                           const int *__restrict__ cols, const T *__restrict__ vals,
+                                           const T *__restrict__ x, T *__restrict__ y, int r0, int nr, int B0, int n)
 {
   extern __shared__ __align__ (16) unsigned char smem[];
   constexpr int VS = 16 / (int) sizeof (T);
   const int bs = BSC ? BSC : bs_rt;
   const int E = bs * bs;
   const int t = threadIdx.x;
-  const int r0 = blockIdx.x * P.rows;
-  const int nr = min (nbr - r0, P.rows);
-  const int B0 = __ldg (row_ptr + r0), B1 = __ldg (row_ptr + r0 + nr);
   const int64_t total_cols = __ldg (row_ptr + nbr), total_vals = total_cols * E;
   T *sv = reinterpret_cast<T *> (smem);
   int *sc = reinterpret_cast<int *> (smem + P.o_cols);
@@ -133,7 +131,6 @@ __global__ void __launch_bounds__ (kThreads, BSC == 3 ? 10 : 8)
   const int K = P.chunk;
   const int slot = t / bs, r = t - slot * bs;
   const int slots = kThreads / bs;
-  const int n = B1 - B0;
 
   for (int p0 = 0; p0 == 0 || p0 < n; p0 += P.cap)
     {
@@ -304,6 +301,94 @@ __global__ void __launch_bounds__ (kThreads, BSC == 3 ? 10 : 8)
     }
 }
 
+// A tile with more than kFullTile times the blocks that a CTA stages at once holds
+// rows far above the average. Where such rows lie together, as in a bordered
+// system, one CTA would walk them all, 4 us for every CTA's fill. So the full tiles
+// of a window of kWindow CTAs are shared out among these by blocks, whole rows at
+// a time; each CTA looks at the window's offsets, which its neighbours read too.
+// At block sizes 3 and 5: from 6 on a warp per block row was no faster on such rows.
+// us, warp per row / a CTA its own tile / this: FP64, 20 000 rows of 7, with 64 rows of
+// 1000 blocks at the end bs 3 91 / 435 / 60, bs 5 259 / 343 / 107, 8 rows of 4000 bs 3
+// 294 / 599 / 101; FP32 bs 5 171 / 259 / 54. Without long rows the second look costs
+// up to 3 %: 150 001 rows of 0-15, bs 3 FP64, 79.9 / 37.1 / 38.3. (Cutting all tiles by
+// blocks, by a search of the offsets: 40.9, bs 12 36.9 -> 39.7.)
+constexpr int kFullTile = 4, kWindow = 32;
+constexpr bool shares_tiles (int bs) { return bs == 3 || bs == 5; }
+
+// Its CTAs: the last window takes the rest too, up to 2 kWindow - 1.
+__device__ __forceinline__ int2 window ()
+{
+  const int last = max (1, (int) gridDim.x / kWindow) - 1, w = min ((int) blockIdx.x / kWindow, last);
+  return make_int2 (w * kWindow, w == last ? (int) gridDim.x : (w + 1) * kWindow);
+}
+
+__device__ __forceinline__ int tile_blocks (const TilePlan &P, int nbr, const int *__restrict__ row_ptr, int tile)
+{
+  const int r0 = min (nbr, tile * P.rows), r1 = min (nbr, r0 + P.rows);
+  return __ldg (row_ptr + r1) - __ldg (row_ptr + r0);
+}
+
+template <typename T, int BSC, int V, bool PAD>
+__device__ __noinline__ void full_tiles (int nbr, int bs_rt, const TilePlan &P, const int *__restrict__ row_ptr,
+                                         const int *__restrict__ cols, const T *__restrict__ vals,
+                                         const T *__restrict__ x, T *__restrict__ y)
+{
+  const int w0 = window ().x, w1 = window ().y;
+  const int me = blockIdx.x - w0, many = w1 - w0;
+  int64_t total = 0;
+  for (int q = w0; q < w1; q++)
+    if (const int n = tile_blocks (P, nbr, row_ptr, q); n > kFullTile * P.cap)
+      total += n;
+  // this CTA's share, counted over the blocks of the window's full tiles
+  const int64_t lo = (total * me + many - 1) / many;
+  const int64_t hi = me + 1 == many ? INT64_MAX : (total * (me + 1) + many - 1) / many;
+  int64_t before = 0;
+  for (int q = w0; q < w1; q++)
+    {
+      const int n = tile_blocks (P, nbr, row_ptr, q);
+      if (n <= kFullTile * P.cap)
+        continue;
+      const int r0 = q * P.rows, nr = min (nbr - r0, P.rows), B0 = __ldg (row_ptr + r0);
+      int beg = 0, end = 0; // rows that begin before the share's ends
+      for (int i0 = 0; i0 < nr; i0 += kThreads)
+        {
+          const int i = i0 + threadIdx.x;
+          const int64_t at = i < nr ? before + __ldg (row_ptr + r0 + i) - B0 : INT64_MAX;
+          beg += __syncthreads_count (i < nr && at < lo);
+          end += __syncthreads_count (i < nr && at < hi);
+        }
+      if (beg < end)
+        {
+          const int b = __ldg (row_ptr + r0 + beg);
+          tile_pass<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y, r0 + beg, end - beg, b,
+                                     __ldg (row_ptr + r0 + end) - b);
+        }
+      before += n;
+    }
+}
+
+template <typename T, int BSC, int V, bool PAD>
+__global__ void __launch_bounds__ (kThreads, BSC == 3 ? 10 : shares_tiles (BSC) ? 9 : 8)
+  tile_kernel (int nbr, int bs_rt, const __grid_constant__ TilePlan P, const int *__restrict__ row_ptr,
+               const int *__restrict__ cols, const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
+{
+  const int r0 = blockIdx.x * P.rows;
+  const int nr = min (nbr - r0, P.rows);
+  const int B0 = __ldg (row_ptr + r0), n = __ldg (row_ptr + r0 + nr) - B0;
+  if constexpr (shares_tiles (BSC))
+    {
+      const int2 w = window ();
+      const int tile = min (w.x + (int) threadIdx.x, w.y - 1);
+      const int a0 = __ldg (row_ptr + tile * P.rows), a1 = __ldg (row_ptr + min (nbr, (tile + 1) * P.rows));
+      if (n <= kFullTile * P.cap)
+        tile_pass<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y, r0, nr, B0, n);
+      if (__syncthreads_or (a1 - a0 > kFullTile * P.cap))
+        full_tiles<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y);
+    }
+  else
+    tile_pass<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y, r0, nr, B0, n);
+}
+
 template <typename T, int BSC, int V>
 int launch (int nbr, int bs, TilePlan P, const int *rp, const int *c, const T *v, const T *x, T *y, cudaStream_t s)
 {
@@ -318,8 +403,6 @@ int launch (int nbr, int bs, TilePlan P, const int *rp, const int *c, const T *v
   P.o_first = P.o_rp + up ((P.rows + 1) * 4);
   P.smem = P.o_first + up ((size_t) (P.cap + P.chunk - 1) / P.chunk * 4);
   const unsigned grid = (unsigned) ((nbr + P.rows - 1) / P.rows);
-  if (P.smem > 48 * 1024)
-    BMFP_CUDA (cudaFuncSetAttribute (tile_kernel<T, BSC, V, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, P.smem));
   tile_kernel<T, BSC, V, PAD><<<grid, kThreads, P.smem, s>>> (nbr, bs, P, rp, c, v, x, y);
   BMFP_LAUNCH_CHECK ();
   return BMFP_SUCCESS;

@@ -273,6 +273,55 @@ def test_row_tiles(lib, orc, cuda, bs, kind, dtype):
         assert np.all(np.abs(y[:n] - orc.bcsr_spmv(rp, c, v, bs, xf[off:])) <= tol)
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("where", ["end", "start", "two windows", "everywhere"])
+@pytest.mark.parametrize("bs", [3, 5])
+def test_row_tiles_share_long_rows_that_lie_together(lib, orc, cuda, bs, where, dtype):
+    """Tiles that hold many times what a CTA stages, at the ends of the matrix, on
+    both sides of a window's edge and all over: every row right; and not much
+    longer than with the same rows spread (one CTA took them one after the
+    other, six times as long)."""
+    import torch
+    rng = np.random.default_rng(bs)
+    n, long_rows, length = 60000, 48, 600
+    base = rng.integers(3, 9, n)
+    slots = 128 // bs
+    cap = max(1, round(20 * 1024 / ((bs * bs * np.dtype(dtype).itemsize + 4) * slots))) * slots
+    times = {}
+    for kind in (where, "spread"):
+        counts = base.copy()
+        window = 32 * int(cap / ((base.sum() + long_rows * length) / n))  # rows
+        at = {"end": np.arange(n - long_rows, n), "start": np.arange(long_rows),
+              "two windows": np.arange(window - 30, window + 18), "everywhere": np.arange(0, n, 997),
+              "spread": np.linspace(0, n - 1, long_rows).astype(int)}[kind]
+        counts[at] = length
+        if kind == "everywhere":
+            counts[at[::7] + 1] = 3000
+            counts[5000:9000] = 0
+        rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+        c = rng.integers(0, n, int(rp[-1])).astype(np.int32)
+        v = rng.uniform(-1, 1, int(rp[-1]) * bs * bs).astype(dtype)
+        x = rng.uniform(-1, 1, n * bs).astype(dtype)
+        d = [dev(a) for a in (rp, c, v, x)]
+        d_y = torch.full((n * bs + GUARD,), float("nan"), dtype=d[3].dtype, device="cuda")
+        t = []
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            bm.bcsr_spmv(bm.BCSR_NATIVE, *d, d_y, bs, n)
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+        times[kind] = min(t)
+        y = d_y.cpu().numpy()
+        assert np.isnan(y[n * bs:]).all()
+        crp, cc, cv = orc.bcsr_to_csr(rp, c, v, bs)
+        tol = spmv_tolerance(orc, crp, cc, cv, x, dtype)
+        assert np.all(np.abs(y[:n * bs] - orc.bcsr_spmv(rp, c, v, bs, x)) <= tol)
+    if where != "everywhere":
+        assert times[where] < 2.5 * times["spread"], times
+
+
 @pytest.mark.parametrize("kind", ["uneven", "empty tail", "one row", "no blocks"])
 @pytest.mark.parametrize("nbr", [1, 7, 1216, 1217, 2432, 2433, 4864, 4865])
 @pytest.mark.parametrize("bs", [16, 32])
