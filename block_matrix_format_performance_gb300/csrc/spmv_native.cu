@@ -411,6 +411,9 @@ int native_lane_candidates (int dtype, int bs, int *out, int max_out)
       out[n++] = g;
   if (bs >= 4 && n < max_out)
     out[n++] = BMFP_LANES_ROW_OWNER;
+  // the rings, which no lane count names
+  if (dtype == BMFP_R64F && bs >= 16 && n < max_out)
+    out[n++] = 0;
   return n;
 }
 

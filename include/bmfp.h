@@ -242,7 +242,8 @@ BMFP_API int bmfp_matrix_spmv (bmfp_matrix_t m, const void *d_x, void *d_y, void
 /* Time candidate lane counts on this matrix (CUDA events, synchronises the
  * stream) and keep the fastest for later bmfp_matrix_spmv calls. x and y are
  * scratch device vectors of the right size. Optional: the default choice is
- * the built-in heuristic. */
+ * the built-in heuristic (chosen_lanes 0 where the fastest kernel is one that no
+ * lane count names: FP64 at block sizes 16 and 32). */
 BMFP_API int bmfp_matrix_autotune (bmfp_matrix_t m, const void *d_x, void *d_y, void *stream,
                                    int *chosen_lanes);
 /* Pin the native kernel's mapping for this handle (values as for

@@ -51,3 +51,21 @@ A = grid_matrix(40)
 s = bm.Solver(A, {precision!r}, stream=STREAM, launch_mode={mode!r}, fallback_fp64=0)
 assert fake.fake_pending(STREAM) == 0, fake.fake_pending(STREAM)
 """)
+
+
+@pytest.mark.parametrize("bs", [16, 32])
+def test_autotuner_can_pick_the_default(fake, bs):
+    """FP64 at block sizes 16 and 32: no explicit lane count names the default
+    kernel, so the autotuner has to time it beside them. Each candidate in turn
+    is made the fastest."""
+    run(fake, f"""
+m = bm.Matrix.from_bcsr(np.array([0, 1], np.int32), np.array([0], np.int32), np.ones({bs * bs}), {bs}, stream=STREAM)
+fake.fake_fast_intervals(-1, -1)
+m.autotune(0x10000, 0x20000, stream=STREAM)
+n, reps = fake.fake_intervals(), 5
+picked = []
+for k in range(0, n, reps):
+    fake.fake_fast_intervals(k, k + reps)
+    picked.append(m.autotune(0x10000, 0x20000, stream=STREAM))
+assert 0 in picked and len(set(picked)) == len(picked) == n // reps, picked
+""")
