@@ -1800,7 +1800,8 @@ int WideEngine::build_sliced (cudaStream_t s)
 
 // The resident iteration kernel's plan, for the auto launch mode: a sliced
 // matrix, no preconditioner or point Jacobi, fewer rows than the persistent
-// kernel's, and vectors that fit the SMs' shared memory beside each other.
+// kernel's, and vectors that fit the SMs' shared memory beside each other. Where
+// its own allocations find no room the graphs run.
 constexpr int kStagedRows = 1408;
 
 int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
@@ -1820,7 +1821,15 @@ int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
     return BMFP_SUCCESS;
   const size_t o_flags = sizeof (unsigned long long) * 2 * kSlotKinds * 2 * kCopies * (size_t) P.grid;
   const size_t o_need = (o_flags + sizeof (unsigned) * kFlagStride * (size_t) P.grid + 15) / 16 * 16;
-  BMFP_CUDA (cudaMalloc (&resident_mem_, o_need + sizeof (int2) * ((size_t) P.grid + 1)));
+  auto give_up = [&] () {
+    cudaGetLastError ();
+    cudaFree (resident_mem_);
+    cudaFree (resident_pub_);
+    resident_mem_ = resident_pub_ = nullptr;
+    return BMFP_SUCCESS;
+  };
+  if (cudaMalloc (&resident_mem_, o_need + sizeof (int2) * ((size_t) P.grid + 1)) != cudaSuccess)
+    return give_up ();
   resident_zero_ = o_need;
   BMFP_CUDA (cudaMemsetAsync (resident_mem_, 0, o_need + sizeof (int2) * ((size_t) P.grid + 1), s));
   P.slots = (unsigned long long *) resident_mem_;
@@ -1847,7 +1856,8 @@ int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
       // p and s as tagged words: a tag beside every four bytes
       const size_t vec = (size_t) S * 2 * (size_t) n_;
       resident_pub_bytes_ = 2 * vec;
-      BMFP_CUDA (cudaMalloc (&resident_pub_, resident_pub_bytes_));
+      if (cudaMalloc (&resident_pub_, resident_pub_bytes_) != cudaSuccess)
+        return give_up ();
       BMFP_CUDA (cudaMemsetAsync (resident_pub_, 0, resident_pub_bytes_, s));
       BMFP_CUDA (cudaStreamSynchronize (s)); // a solve on another stream would meet it
       P.pub[0] = (unsigned long long *) resident_pub_;
@@ -1859,7 +1869,7 @@ int WideEngine::plan_resident (int dev, int sms, cudaStream_t s)
   BMFP_CUDA (cudaFuncSetAttribute (fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   BMFP_CUDA (cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, fn, P.threads, (size_t) P.smem));
   if ((int64_t) per_sm * sms < P.grid)
-    return BMFP_SUCCESS; // the graph then
+    return give_up ();
   resident_ = P;
   iterate_ = fn;
   return BMFP_SUCCESS;

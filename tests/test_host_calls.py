@@ -69,3 +69,31 @@ for k in range(0, n, reps):
     picked.append(m.autotune(0x10000, 0x20000, stream=STREAM))
 assert 0 in picked and len(set(picked)) == len(picked) == n // reps, picked
 """)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_no_room_for_the_resident_kernel_leaves_the_graphs(fake, precision):
+    """Each allocation of a solver's creation fails in turn. The ones that only
+    the auto mode makes (the sliced copy, and the words, flags and published
+    vectors of its kernel) are not needed for a solve."""
+    run(fake, f"""
+A = grid_matrix(40)
+def create(mode, fail):
+    fake.fake_fail_malloc(fail)
+    s = bm.Solver(A, {precision!r}, stream=STREAM, launch_mode=mode)
+    s.close()
+    return fake.fake_mallocs()
+def survives(mode, k):
+    graphs = fake.fake_graphs()
+    try:
+        create(mode, k)
+    except bm.BmfpError:
+        return False
+    assert fake.fake_graphs() == graphs + 1, (mode, k)
+    return True
+counts = {{mode: create(mode, -1) for mode in ("auto", "graph")}}
+extra = counts["auto"] - counts["graph"]
+assert extra >= 1, counts
+spare = {{mode: sum(survives(mode, k) for k in range(counts[mode])) for mode in counts}}
+assert spare["auto"] == spare["graph"] + extra, (counts, spare)
+""")
