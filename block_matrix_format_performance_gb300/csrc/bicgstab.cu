@@ -1644,6 +1644,7 @@ int WideEngine::init (const bmfp_matrix_s *A, int precond, int chunk, cudaStream
   // 2 M rows 251.3 / 234.0; at 4 CTAs per SM and 64 registers the
   // persistent kernel spilled and took 84.2 / 142.2 / 234.0).
   iterate_ = nullptr;
+  auto_ = launch_mode == BMFP_LAUNCH_AUTO;
   int cps = std::max (1, std::min (ctas_per_sm, 8));
   if (launch_mode == BMFP_LAUNCH_PERSISTENT || (launch_mode == BMFP_LAUNCH_AUTO && n_ >= kPersistentRows))
     {
@@ -1980,6 +1981,10 @@ int WideEngine::start (bool zero, const void *c, double tol, int max_iter, doubl
   const double eps = replace_ ? unit_roundoff (dtype_) : 0.0;
   c_ = c;
   from_zero_ = zero;
+  tol_ = tol;
+  max_iter_ = max_iter;
+  iter0_ = iter0;
+  new_shadow_ = new_shadow;
   if (dtype_ == BMFP_R64F)
     {
       const Args<double> a
@@ -2028,9 +2033,9 @@ __global__ void stop_kernel (DevState *st)
 }
 } // namespace
 
-// A barrier of the persistent kernel gave up: the barrier words may hold a
+// A wait of the persistent or resident kernel gave up: its words may hold a
 // partial count, so the state (and the partials) are cleared (the next solve
-// starts a new run) and the solve fails.
+// starts a new run) and the solve fails, unless the mode was the library's choice.
 int WideEngine::barrier_fault (cudaStream_t s)
 {
   BMFP_CUDA (cudaStreamSynchronize (s));
@@ -2042,6 +2047,24 @@ int WideEngine::barrier_fault (cudaStream_t s)
     BMFP_CUDA (cudaMemsetAsync (resident_pub_, 0, resident_pub_bytes_, s));
   BMFP_CUDA (cudaStreamSynchronize (s));
   return fail (BMFP_ERROR_TIMEOUT, "a grid barrier of the iteration kernel gave up waiting");
+}
+
+// After a wait that gave up under the auto mode: the graphs take this run again
+// from its start (x is written at its end only), and all later ones. `last` is a
+// state of the run, for what a restart keeps of the runs before it.
+int WideEngine::run_again_as_graphs (const DevState &last, cudaStream_t s)
+{
+  iterate_ = nullptr;
+  resident_ = ResidentPlan ();
+  cudaFree (resident_mem_);
+  cudaFree (resident_pub_);
+  resident_mem_ = resident_pub_ = nullptr;
+  const int rc = capture (capture_stream_);
+  if (rc != BMFP_SUCCESS)
+    return rc;
+  if (from_zero_)
+    return start (true, c_, tol_, max_iter_, -1.0, 0, new_shadow_, s);
+  return start (false, c_, tol_, max_iter_, last.norm_b, iter0_ >= 0 ? iter0_ : last.iter, new_shadow_, s);
 }
 
 int WideEngine::run (cudaStream_t s, DevState *out, void *d_snap, double *snap_rr, int stall)
@@ -2073,7 +2096,22 @@ int WideEngine::run (cudaStream_t s, DevState *out, void *d_snap, double *snap_r
           BMFP_CUDA (cudaEventSynchronize (ev_[(k - 1) & 1]));
           const DevState &h = h_state_[(k - 1) & 1];
           if (h.fault)
-            return barrier_fault (s);
+            {
+              const DevState last = h;
+              int rc = barrier_fault (s);
+              if (rc == BMFP_ERROR_TIMEOUT && auto_)
+                rc = run_again_as_graphs (last, s);
+              if (rc != BMFP_SUCCESS)
+                return rc;
+              best = snap_at = mark = INFINITY; // no copy of the aborted run counts
+              if (snap_rr)
+                *snap_rr = INFINITY;
+              snap_k = -1;
+              mark_it = 0;
+              stopping = false;
+              k = -1;
+              continue;
+            }
           if (snap_k == k - 1)
             *snap_rr = snap_at = h.rr;
           if (h.done)

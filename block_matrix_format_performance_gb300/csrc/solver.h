@@ -170,6 +170,7 @@ private:
   int launch_phase (int phase, cudaStream_t stream);
   int launch_iterations (cudaStream_t stream);
   int barrier_fault (cudaStream_t stream);
+  int run_again_as_graphs (const DevState &last, cudaStream_t stream);
   int start (bool zero, const void *c, double tol, int max_iter, double norm_b, int iter0, bool new_shadow,
              cudaStream_t s);
 
@@ -185,6 +186,10 @@ private:
   int spmv_kind_ = 0;
   double cA_ = 0.0; // entries per row * ||A||_inf (replacement bound)
   const void *c_ = nullptr; // right-hand side of the current run
+  double tol_ = 0.0;        // and its other arguments (start)
+  int max_iter_ = 0, iter0_ = 0;
+  bool new_shadow_ = false;
+  bool auto_ = false; // the launch mode is the library's choice
   void *x_ = nullptr, *r_ = nullptr, *rh_ = nullptr, *p_ = nullptr, *v_ = nullptr;
   void *q_ = nullptr, *s_ = nullptr, *z_ = nullptr, *t_ = nullptr, *P_ = nullptr;
   void *g_ = nullptr, *xp_ = nullptr;

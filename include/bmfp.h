@@ -284,7 +284,9 @@ enum bmfp_launch_mode
                                  and bs = 2 without block Jacobi, one cooperative kernel per
                                  iterations_per_graph iterations that keeps the Krylov vectors in
                                  shared memory, where they fit (about 600 000 rows in FP64) and
-                                 check_true_residual is 1; else graphs */
+                                 check_true_residual is 1; else graphs. A cooperative kernel whose
+                                 wait for its other CTAs gives up (4 s) leaves the solve, and later
+                                 ones, to the graphs */
   BMFP_LAUNCH_GRAPH = 1,      /* a CUDA graph of five phase kernels per iteration */
   BMFP_LAUNCH_PERSISTENT = 2  /* one cooperative kernel per iterations_per_graph iterations, the
                                  phases separated by grid barriers, over min(ctas_per_sm, 3) CTAs

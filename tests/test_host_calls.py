@@ -97,3 +97,24 @@ assert extra >= 1, counts
 spare = {{mode: sum(survives(mode, k) for k in range(counts[mode])) for mode in counts}}
 assert spare["auto"] == spare["graph"] + extra, (counts, spare)
 """)
+
+
+def test_auto_mode_returns_to_the_graphs_after_a_timeout(fake):
+    """A cooperative kernel whose waits give up: the auto mode solves again with
+    the graphs and stays with them; a caller who asked for the kernel is told."""
+    run(fake, """
+b, x = np.zeros(3200), np.empty(3200)
+A = grid_matrix(40)
+fake.fake_cooperative_fault(1)
+s = bm.Solver(A, "fp64", stream=STREAM)
+graphs = fake.fake_graphs()
+for _ in range(2):
+    assert s.solve(b, x, stream=STREAM)["status"] == bm.SUCCESS
+    assert fake.fake_graphs() == graphs + 1
+p = bm.Solver(A, "fp64", stream=STREAM, launch_mode="persistent")
+try:
+    p.solve(b, x, stream=STREAM)
+    assert False
+except bm.BmfpError as e:
+    assert e.status == bm.ERROR_TIMEOUT, e
+""")
