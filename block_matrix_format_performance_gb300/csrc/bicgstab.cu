@@ -1739,6 +1739,19 @@ bool streams (int dtype, int b, size_t bytes, int64_t n)
 // padding stays below an eighth (a structured grid's below 1 %) and it takes at
 // most a quarter of the free memory; the products walk the block rows
 // otherwise.
+// Blocks of the copy at most, padding included.
+size_t sliced_blocks (int64_t nnz) { return (size_t) (nnz + nnz / 8 + 1024); }
+
+size_t sliced_bytes (const bmfp_matrix_s *A, const bmfp_solver_options &o)
+{
+  const size_t B = A->bs == 2 ? 2 : 1;
+  if (A->bs > 2 || o.check_true_residual == 0)
+    return 0;
+  const size_t rows = (size_t) A->n_rows * B, entries = sliced_blocks (A->nnz);
+  auto copy = [&] (size_t S) { return entries * (B * B * S + sizeof (int)) + sizeof (int) * (rows / kSlice + 2); };
+  return (o.precision != BMFP_SOLVE_FP32 ? copy (8) : 0) + (o.precision != BMFP_SOLVE_FP64 ? copy (4) : 0);
+}
+
 int WideEngine::build_sliced (cudaStream_t s)
 {
   const int nbr = A_->n_rows;
@@ -1765,7 +1778,7 @@ int WideEngine::build_sliced (cudaStream_t s)
   size_t mem_free = 0, mem_total = 0;
   if (e == cudaSuccess)
     e = cudaMemGetInfo (&mem_free, &mem_total);
-  if (e == cudaSuccess && o_off < mem_free / 4 && blocks <= (size_t) (A_->nnz + A_->nnz / 8 + 1024) && total <= INT32_MAX
+  if (e == cudaSuccess && o_off < mem_free / 4 && blocks <= sliced_blocks (A_->nnz) && total <= INT32_MAX
       && cudaMalloc (&svals_, o_off + sizeof (int) * ((size_t) ns + 1)) == cudaSuccess)
     {
       scols_ = (int *) ((char *) svals_ + B * B * S * blocks);

@@ -50,6 +50,7 @@ struct Request
   bmfp_solve_info info{};
   bool done = false;
   bool wide = false;
+  bool plain = false; // a wide one without the sliced copies (request_bytes)
   // device slices (inside the micro-batch's allocation)
   double *d_b = nullptr, *d_x = nullptr, *w64 = nullptr;
   float *w32 = nullptr;
@@ -155,10 +156,18 @@ struct bmfp_server_s
 
 namespace
 {
-size_t request_bytes (const bmfp_server_s *sv, int64_t n, bool wide)
+// *plain: a whole-GPU request that fits the budget only without its lane's sliced
+// copies of the matrix, which its solver then leaves out.
+size_t request_bytes (const bmfp_server_s *sv, const bmfp_matrix_s *A, int64_t n, bool wide, bool *plain)
 {
+  *plain = false;
   if (wide)
-    return (size_t) n * 8 * 15; // solver vectors (work and Krylov) + b, x
+    {
+      const size_t vectors = (size_t) n * 8 * 15; // solver vectors (work and Krylov) + b, x
+      const size_t copies = sliced_bytes (A, sv->opts.solver);
+      *plain = vectors + copies > sv->opts.hbm_budget_bytes;
+      return *plain ? vectors : vectors + copies;
+    }
   size_t b = align256 (n * 8) * 2 + align256 (n * 8 * kBatchW64); // b, x, FP64 work vectors
   if (sv->opts.solver.precision != BMFP_SOLVE_FP64)
     b += align256 (n * 4 * 8); // 8 FP32 work vectors
@@ -505,7 +514,7 @@ void wide_main (bmfp_server_s *sv, int lane)
           // Lanes share the GPU with the batched solver and each other: a
           // persistent kernel would hold every SM while it runs.
           o.launch_mode = BMFP_LAUNCH_GRAPH;
-          rc = bmfp_solver_create (&solver, const_cast<bmfp_matrix_s *> (r->A), &o, stream);
+          rc = create_solver (&solver, const_cast<bmfp_matrix_s *> (r->A), &o, r->plain, stream);
           if (rc == BMFP_SUCCESS)
             sv->wide_solvers[key] = solver;
         }
@@ -664,7 +673,7 @@ int bmfp_server_submit (bmfp_server_t sv, bmfp_matrix_t A, const double *h_b, do
   r->b.assign (h_b, h_b + r->n);
   r->h_x = h_x;
   r->wide = r->n > sv->opts.wide_threshold_rows;
-  r->bytes = request_bytes (sv, r->n, r->wide);
+  r->bytes = request_bytes (sv, A, r->n, r->wide, &r->plain);
   r->t_submit = Clock::now ();
   r->info.status = BMFP_PENDING;
   if (r->bytes > sv->opts.hbm_budget_bytes)

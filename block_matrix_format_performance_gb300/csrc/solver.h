@@ -234,6 +234,11 @@ int raw_solve_grid (int64_t n, int *grid);
 // The persistent kernel's grid barrier made to time out on purpose (a wait
 // for one CTA more than the grid holds) after limit_s: reports the fault flag
 // the timed-out CTAs set and how long the launch took.
+// bmfp_solver_create, with the sliced copies left out where `plain` says so; and
+// the bytes of those copies at most (none where the engine makes none).
+int create_solver (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_options *opts, bool plain, void *stream);
+size_t sliced_bytes (const bmfp_matrix_s *A, const bmfp_solver_options &opts);
+
 int barrier_selftest (double limit_s, int *fault, double *elapsed_s, cudaStream_t s);
 int resident_selftest (double limit_s, int *faults, cudaStream_t s);
 int raw_jacobi (const RawSolve &b, cudaStream_t stream);

@@ -344,30 +344,8 @@ int probe_fp32 (bmfp_solver_s *sv, cudaStream_t s, bool *fp64_only)
 }
 } // namespace
 
-extern "C" {
-
-void bmfp_solver_options_init (bmfp_solver_options *o)
-{
-  if (!o)
-    return;
-  o->precision = BMFP_SOLVE_FP64;
-  o->preconditioner = BMFP_PRECOND_NONE;
-  o->tolerance = 1e-10;
-  o->max_iterations = 100000;
-  o->check_true_residual = 1;
-  o->inner_tolerance = 1e-4;
-  o->inner_max_iterations = 1000;
-  o->max_refinements = 30;
-  o->fallback_fp64 = 1;
-  o->iterations_per_graph = 16;
-  o->ctas_per_sm = 4;
-  o->inner_stall_iterations = 64;
-  o->residual_replacement = 1;
-  o->launch_mode = BMFP_LAUNCH_AUTO;
-}
-
-int bmfp_solver_create (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_options *opts,
-                        void *stream)
+int bmfp::create_solver (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_options *opts, bool plain,
+                         void *stream)
 {
   if (!out || !A)
     return fail (BMFP_ERROR_INVALID_VALUE, "null argument");
@@ -404,7 +382,7 @@ int bmfp_solver_create (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_o
   // Without the true-residual check (the reference's stopping rule) a solve
   // takes the iterations of the allocation-free entry point, which has no
   // room for a copy of the matrix: the same kernels on the same arrays.
-  const bool plain = o.check_true_residual == 0;
+  plain = plain || o.check_true_residual == 0;
   int rc = BMFP_SUCCESS;
   const bmfp_matrix_s *A32 = A;
   if (o.precision != BMFP_SOLVE_FP64 && A->dtype == BMFP_R64F)
@@ -447,6 +425,34 @@ int bmfp_solver_create (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_o
     }
   *out = sv.release ();
   return BMFP_SUCCESS;
+}
+
+extern "C" {
+
+void bmfp_solver_options_init (bmfp_solver_options *o)
+{
+  if (!o)
+    return;
+  o->precision = BMFP_SOLVE_FP64;
+  o->preconditioner = BMFP_PRECOND_NONE;
+  o->tolerance = 1e-10;
+  o->max_iterations = 100000;
+  o->check_true_residual = 1;
+  o->inner_tolerance = 1e-4;
+  o->inner_max_iterations = 1000;
+  o->max_refinements = 30;
+  o->fallback_fp64 = 1;
+  o->iterations_per_graph = 16;
+  o->ctas_per_sm = 4;
+  o->inner_stall_iterations = 64;
+  o->residual_replacement = 1;
+  o->launch_mode = BMFP_LAUNCH_AUTO;
+}
+
+int bmfp_solver_create (bmfp_solver_t *out, bmfp_matrix_t A, const bmfp_solver_options *opts,
+                        void *stream)
+{
+  return bmfp::create_solver (out, A, opts, false, stream);
 }
 
 int bmfp_solver_solve (bmfp_solver_t sv, const void *d_b, void *d_x, bmfp_solve_info *info_out,

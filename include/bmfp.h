@@ -435,7 +435,9 @@ typedef struct bmfp_server_s *bmfp_server_t;
 
 typedef struct bmfp_server_options
 {
-  size_t hbm_budget_bytes;     /* device bytes for admitted requests (default 120 GiB) */
+  size_t hbm_budget_bytes;     /* device bytes for admitted requests (default 120 GiB); a whole-GPU
+                                  request counts its solver's sliced copies of a CSR or bs = 2 matrix,
+                                  and runs without them where it fits only so */
   int max_in_flight;           /* requests on the device at once (default 4096) */
   int max_batch;               /* requests per micro-batch launch (default 64) */
   int streams;                 /* concurrent micro-batches (default 8) */

@@ -83,6 +83,29 @@ def test_admission_respects_the_budget(problems):
         assert rel_residual(rp, c, v, b, x) < 1e-10
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_whole_gpu_requests_count_their_copies_of_the_matrix(problems, precision):
+    """A lane's solver keeps sliced copies of the matrix beside its vectors. The
+    budget counts them, and a request that fits only without them is solved
+    without them."""
+    m, rp, c, v, _ = problems[7]
+    vectors = 15 * 8 * m.rows
+    # 36 bytes a block in FP64, 20 more in mixed precision, at most an eighth and
+    # 1024 blocks of padding
+    copies = c.size * (36 if precision == "fp64" else 56)
+    peaks = []
+    for budget in (120 << 30, vectors + copies // 2):
+        srv = bm.Server(precision, tol=1e-10, wide_threshold_rows=1000, hbm_budget_bytes=budget)
+        x = np.zeros(m.rows)
+        b = loads(m.rows, 7)
+        info = srv.wait(srv.submit(m, b, x))
+        peaks.append(srv.stats()["peak_bytes"])
+        srv.close()
+        assert info["status"] == bm.SUCCESS and rel_residual(rp, c, v, b, x) < 1e-10
+    assert vectors + copies <= peaks[0] <= vectors + 1.13 * copies + (1100 + m.rows) * 56
+    assert peaks[1] == vectors
+
+
 def test_request_larger_than_budget_is_refused(problems):
     m = problems[7][0]
     srv = bm.Server("fp64", hbm_budget_bytes=1024)
