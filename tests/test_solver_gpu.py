@@ -706,6 +706,27 @@ def test_auto_mode_at_the_ends_of_the_exponents(lib, orc, cuda, grid, power):
     A.close()
 
 
+@pytest.mark.parametrize("mode", ["auto", "graph"])
+@pytest.mark.parametrize("grid", [(40, 30), (200, 50)])
+def test_infinite_right_hand_side_breaks_down_and_leaves_no_trace(lib, cuda, grid, mode):
+    """Infinities leave the exponents that are summed as integers. The solve ends
+    as a breakdown, and the solver's next one has the bits of a fresh solver."""
+    import torch
+    rp, c, v = shifted_q4(*grid)
+    n = 2 * grid[0] * grid[1]
+    A = bm.Matrix.from_bcsr(rp, c, v, 2)
+    b = dev(np.random.default_rng(2).uniform(-1, 1, n))
+    bad = b.clone()
+    bad[n // 2] = float("inf")
+    fresh, again = torch.empty_like(b), torch.empty_like(b)
+    assert bm.Solver(A, "fp64", tol=1e-12, launch_mode=mode).solve(b, fresh)["status"] == bm.SUCCESS
+    s = bm.Solver(A, "fp64", tol=1e-12, launch_mode=mode)
+    assert s.solve(bad, again)["status"] == bm.ERROR_BREAKDOWN
+    assert s.solve(b, again)["status"] == bm.SUCCESS
+    assert torch.equal(fresh.view(torch.int64), again.view(torch.int64))
+    A.close()
+
+
 def test_auto_mode_solves_on_separate_streams(lib, cuda):
     """Four auto solves at once from four threads on four streams, staged and
     unstaged: each has the bits of the same solve run alone."""

@@ -274,6 +274,30 @@ def test_row_tiles(lib, orc, cuda, bs, kind, dtype):
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("which", ["values", "columns"])
+@pytest.mark.parametrize("bs", [3, 12, 16])
+def test_misaligned_arrays_where_aligned_ones_are_staged(lib, orc, cuda, bs, which, dtype):
+    """Values or columns one element off a 16-byte boundary, at sizes whose aligned
+    arrays take the row tiles or (bs 16) the rings: those copy 16 bytes at a time."""
+    import torch
+    rp, c, v, nbc = tiled_bcsr(bs, dtype, bs, "uneven")
+    n = (rp.size - 1) * bs
+    x = np.random.default_rng(bs).uniform(-1, 1, nbc * bs).astype(dtype)
+    d_c, d_v = dev(c), dev(v)
+    if which == "values":
+        d_v = dev(np.concatenate([v[:1], v]))[1:]
+    else:
+        d_c = dev(np.concatenate([c[:1], c]))[1:]
+    d_y = torch.full((n + GUARD,), float("nan"), dtype=d_v.dtype, device="cuda")
+    bm.bcsr_spmv(bm.BCSR_NATIVE, dev(rp), d_c, d_v, dev(x), d_y, bs, nbc)
+    y = d_y.cpu().numpy()
+    assert np.isnan(y[n:]).all()
+    crp, cc, cv = orc.bcsr_to_csr(rp, c, v, bs)
+    tol = spmv_tolerance(orc, crp, cc, cv, x, dtype)
+    assert np.all(np.abs(y[:n] - orc.bcsr_spmv(rp, c, v, bs, x)) <= tol)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("where", ["end", "start", "two windows", "everywhere"])
 @pytest.mark.parametrize("bs", [3, 5])
 def test_row_tiles_share_long_rows_that_lie_together(lib, orc, cuda, bs, where, dtype):
