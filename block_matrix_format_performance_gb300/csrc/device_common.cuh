@@ -64,6 +64,18 @@ __device__ __forceinline__ void ld_cached2 (const double *p, double &a, double &
 template <typename T> __device__ __forceinline__ T ld_stream (const T *p) { return __ldcs (p); }
 template <typename T> __device__ __forceinline__ T ld_cached (const T *p) { return __ldg (p); }
 
+// Asynchronous copies to shared memory: 16 bytes (zeros behind the first `bytes`),
+// the end of a group of them, and the wait until at most N groups are on their way.
+__device__ __forceinline__ void cp_async16 (uint32_t dst, const void *src, int bytes)
+{
+  asm volatile ("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit () { asm volatile ("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait ()
+{
+  asm volatile ("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // How the row routines load the vector they multiply.
 // XNc: the read-only path, for a vector no thread of the running kernel writes.
 struct XNc

@@ -157,7 +157,12 @@ __global__ void __launch_bounds__ (kThreads)
 // warp w takes the w-th row of each. us, by 32 lanes a row / by the warp of the
 // row's own group / this: 200 000 rows of 18, FP64, 8 rows of 100 000 entries at the
 // end 1641 / 11690 / 1545, 64 of 20 000 408 / 2510 / 337; the 1000x250 elasticity operator,
-// without long rows, 215 / 36.8 / 36.9. (A warp looking at rows W apart instead, no
+// without long rows, 215 / 36.8 / 36.9. The line lies where the warp starts to pay
+// (four million entries, 1 % of the rows long, us by lines of 8 G + 24, 16 G + 48, 32 G +
+// 96, 64 G + 192 and none: FP64, rows of 5 with 100 entries in the long ones 37 / 37 / 70 /
+// 70 / 71, 300 53 / 53 / 53 / 140 / 140; rows of 18, 100 29 / 31 / 31 / 31 / 31, 200 32 / 32 /
+// 41 / 41 / 41, 400 38 / 38 / 38 / 63 / 63; rows of 40, 500 39 / 39 / 38 / 44 / 44; FP32 alike,
+// but rows of 18 with 100 19 / 17.5 / 17.5 / 17.5 / 17.6). (A warp looking at rows W apart instead, no
 // barrier: 37.9, and rows of 5 in FP32 8.9 -> 11.9.)
 template <typename T, int G>
 __global__ void __launch_bounds__ (kThreads)
@@ -334,8 +339,9 @@ int native_bcsr_typed (int nbr, int bs, int64_t nnzb, const int *rp, const int *
     }
   if (bs <= 32)
     {
-      // Row tiles, except at bs 9 in FP32, where the warp per block row is
-      // level with them (35 against 35 us on rows of 0-15 blocks).
+      // Row tiles, except at bs 9 in FP32, where they pay from some 50 000 block
+      // rows up only (us, warp per block row / tiles: 20 000 rows of 0-15 blocks
+      // 18.9 / 20.8, 50 000 37.0 / 36.9, 150 000 94 / 88; 150 000 rows of 7 90 / 78).
       const bool staged = ((reinterpret_cast<uintptr_t> (v) | reinterpret_cast<uintptr_t> (c)) & 15u) == 0;
       if (!flat_bs (bs) && staged && !(bs == 9 && sizeof (T) == 4))
         {

@@ -28,21 +28,6 @@ namespace
 {
 constexpr int kThreads = 128;
 
-__device__ __forceinline__ void cp_async16 (uint32_t dst, const void *src, int bytes)
-{
-  asm volatile ("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-
-template <int N> __device__ __forceinline__ void cp_async_wait ()
-{
-  asm volatile ("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit ()
-{
-  asm volatile ("cp.async.commit_group;" ::: "memory");
-}
-
 // Stages of the ring, and bytes of one warp's stage: its 32 / BS blocks, then
 // their x. Two CTAs of four warps per SM: two warps to an FP64 pipe.
 template <int BS> constexpr int ring_depth () { return BS == 32 ? 3 : 6; }
@@ -122,14 +107,14 @@ __global__ void __launch_bounds__ (kThreads)
         for (int i = 0; i < P; i++)
           {
             const int q = i * BS + r; // the group reads BS pieces side by side
-            cp_async16 (s + (uint32_t) ((g * BS * P + place<BS> (q / P, q % P)) * 16), b + q * 2, 16);
+            dev::cp_async16 (s + (uint32_t) ((g * BS * P + place<BS> (q / P, q % P)) * 16), b + q * 2, 16);
           }
         if (r < P)
-          cp_async16 (s + (uint32_t) (32 * BS * 8 + (g * P + r) * 16), x + (size_t) col * BS + r * 2, 16);
+          dev::cp_async16 (s + (uint32_t) (32 * BS * 8 + (g * P + r) * 16), x + (size_t) col * BS + r * 2, 16);
         if (j + 1 < n)
           col = __ldg (c + j + 1);
       }
-    cp_async_commit ();
+    dev::cp_async_commit ();
   };
 #pragma unroll
   for (int j = 0; j < D - 1; j++)
@@ -153,7 +138,7 @@ __global__ void __launch_bounds__ (kThreads)
   for (int j = 0; j < steps; j++)
     {
       copy (j + D - 1);
-      cp_async_wait<D - 1> ();
+      dev::cp_async_wait<D - 1> ();
       __syncwarp ();
       if (j < n)
         {

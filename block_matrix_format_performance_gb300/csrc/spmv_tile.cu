@@ -1,4 +1,5 @@
-// Row-tile sparse products: y = A x for CSR and for BCSR with any block size.
+// Row-tile sparse products: y = A x for BCSR at block sizes from 3 to 32 that are no
+// power of two.
 //
 // A CTA owns a tile of consecutive block rows, whose values and block columns
 // are two contiguous runs. It copies them into shared memory with 16-byte
@@ -28,16 +29,6 @@ namespace
 {
 constexpr int kThreads = 128;
 constexpr int kMaxRows = 1024; // block rows per CTA at most
-
-__device__ __forceinline__ void cp_async16 (uint32_t dst, const void *src, int bytes)
-{
-  asm volatile ("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all ()
-{
-  asm volatile ("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
 
 template <typename T, int V> struct Pack
 {
@@ -144,14 +135,14 @@ __device__ __forceinline__ void tile_pass (int nbr, int bs_rt, const TilePlan &P
             {
               const int64_t e = ea + (int64_t) j * VS;
               const int left = (int) min ((int64_t) VS, total_vals - e);
-              cp_async16 (sv_a + (PAD ? j + j / 8 : j) * 16, vals + e, left * (int) sizeof (T));
+              dev::cp_async16 (sv_a + (PAD ? j + j / 8 : j) * 16, vals + e, left * (int) sizeof (T));
             }
           const int64_t ca = b0 & ~(int64_t) 3;
           const int nc = (int) ((b0 + nb - ca + 3) / 4);
           for (int j = t; j < nc; j += kThreads)
             {
               const int64_t e = ca + j * 4;
-              cp_async16 (sc_a + j * 16, cols + e, (int) min ((int64_t) 4, total_cols - e) * 4);
+              dev::cp_async16 (sc_a + j * 16, cols + e, (int) min ((int64_t) 4, total_cols - e) * 4);
             }
         }
       if (p0 == 0)
@@ -168,7 +159,8 @@ __device__ __forceinline__ void tile_pass (int nbr, int bs_rt, const TilePlan &P
             for (int q = (lo + K - 1) / K; q * K < hi; q++)
               first[q] = i;
         }
-      cp_async_wait_all ();
+      dev::cp_async_commit ();
+      dev::cp_async_wait<0> ();
       __syncthreads ();
       const int off = (int) ((((int64_t) B0 + p0) * E) & (VS - 1));
       const int *scb = sc + ((B0 + p0) & 3);

@@ -327,7 +327,11 @@ typedef struct bmfp_solver_options
                                auto mode's shared-memory kernel has a grid of its own. The
                                cooperative kernels hold the SMs they run on for a launch, so
                                other work waits for them (the server's lanes, which share the
-                               GPU with the batched solver, use graphs) */
+                               GPU with the batched solver, use graphs). Several threads that
+                               solve systems of 50 000 to 150 000 rows at once may do better
+                               with GRAPH: 80 000 rows in FP64, us per solve with 1, 2, 4 and 8
+                               threads 3840, 3800, 3650, 3620, as graphs 5700, 3900, 3020, 2960
+                               (20 000 rows 1850, 1040, 780, 760 and 3700, 2000, 1100, 780) */
 } bmfp_solver_options;
 
 typedef struct bmfp_solve_info
@@ -352,7 +356,10 @@ typedef struct bmfp_solver_s *bmfp_solver_t;
  * 30 refinements, FP64 fallback on, 16 iterations per graph. */
 BMFP_API void bmfp_solver_options_init (bmfp_solver_options *opts);
 /* Allocate the Krylov vectors and capture the iteration graph. The matrix must
- * be square and must outlive the solver (for MIXED it must be FP64). This call
+ * be square and must outlive the solver (for MIXED it must be FP64). The solver
+ * may multiply by copies of the matrix made here (sliced for CSR and bs = 2, FP32
+ * for FP32 and MIXED, the diagonal's inverses): a matrix whose values change needs
+ * a new solver. This call
  * synchronises the stream; the reference constructor's 80 %-of-memory guard
  * (bicgstab.cu:41-42) becomes BMFP_ERROR_OUT_OF_MEMORY from the allocations.
  * MIXED with fallback_fp64: creation probes the matrix once (the FP32
