@@ -237,7 +237,7 @@ constexpr int kSlice = 32;
 // one CTA per SM, 5 blocks 64 / 73 / 55, 8 blocks 81 / 92 / 76).
 // A copy larger than L2 is read evict-first, columns included (Stream).
 // 2000x500 Q4 grid, FP64, phases 2 and 4 by block rows and by slices: 84.5 and
-// 88.4 us -> 72.8 and 81.1 us (FP64 pipe 74 % -> 82 % busy, its work alone 61
+// 88.4 us -> 74.9 and 80.3 us (FP64 pipe 74 % -> 80 % busy, its work alone 61
 // and 64 us).
 template <typename T, int B, class XL = dev::XNc> struct SellOp
 {
