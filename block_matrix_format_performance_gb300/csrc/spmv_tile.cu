@@ -298,14 +298,16 @@ __device__ __forceinline__ void tile_pass (int nbr, int bs_rt, const TilePlan &P
 // system, one CTA would walk them all, 4 us for every CTA's fill. So the full tiles
 // of a window of kWindow CTAs are shared out among these by blocks, whole rows at
 // a time; each CTA looks at the window's offsets, which its neighbours read too.
-// At block sizes 3 and 5: from 6 on a warp per block row was no faster on such rows.
-// us, warp per row / a CTA its own tile / this: FP64, 20 000 rows of 7, with 64 rows of
-// 1000 blocks at the end bs 3 91 / 435 / 60, bs 5 259 / 343 / 107, 8 rows of 4000 bs 3
-// 294 / 599 / 101; FP32 bs 5 171 / 259 / 54. Without long rows the second look costs
-// up to 3 %: 150 001 rows of 0-15, bs 3 FP64, 79.9 / 37.1 / 38.3. (Cutting all tiles by
-// blocks, by a search of the offsets: 40.9, bs 12 36.9 -> 39.7.)
+// At block size 3 only. us, warp per row / a CTA its own tile / shared, FP64, 20 000 rows of
+// 7 with 64 rows of 1000 blocks at the end: bs 3 91 / 435 / 60, bs 5 259 / 343 / 107, bs 6
+// 322 / 355 / 132, bs 7 480 / 332 / -, more at larger sizes; 8 rows of 4000, bs 3 294 / 599 / 101.
+// Other matrices pay for it (us, own tile / shared: bs 3 FP64, 150 001 rows of 0-15 37.1 /
+// 38.1, 100 000 rows of 7 22.6 / 23.0, 20 000 rows of 7 9.1 / 9.9, FP32 within 2 %; bs 5, 42 000
+// rows of 6, 21.4 / 22.2), which a loss of 4.8 times is worth and one of a
+// third at most is not. (Cutting all tiles by blocks, by a search of the offsets: 40.9, and
+// bs 12 36.9 -> 39.7.)
 constexpr int kFullTile = 4, kWindow = 32;
-constexpr bool shares_tiles (int bs) { return bs == 3 || bs == 5; }
+constexpr bool shares_tiles (int bs) { return bs == 3; }
 
 // Its CTAs: the last window takes the rest too, up to 2 kWindow - 1.
 __device__ __forceinline__ int2 window ()
@@ -360,25 +362,34 @@ __device__ __noinline__ void full_tiles (int nbr, int bs_rt, const TilePlan &P, 
 }
 
 template <typename T, int BSC, int V, bool PAD>
-__global__ void __launch_bounds__ (kThreads, BSC == 3 ? 10 : shares_tiles (BSC) ? 9 : 8)
-  tile_kernel (int nbr, int bs_rt, const __grid_constant__ TilePlan P, const int *__restrict__ row_ptr,
-               const int *__restrict__ cols, const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
+__global__ void __launch_bounds__ (kThreads, 8)
+  tile_kernel (int nbr, int bs_rt, TilePlan P, const int *__restrict__ row_ptr, const int *__restrict__ cols,
+               const T *__restrict__ vals, const T *__restrict__ x, T *__restrict__ y)
+{
+  const int r0 = blockIdx.x * P.rows;
+  const int nr = min (nbr - r0, P.rows);
+  const int B0 = __ldg (row_ptr + r0), B1 = __ldg (row_ptr + r0 + nr);
+  tile_pass<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y, r0, nr, B0, B1 - B0);
+}
+
+// The same with full tiles shared out (P stays where it is: full_tiles takes its
+// address).
+template <typename T, int BSC, int V, bool PAD>
+__global__ void __launch_bounds__ (kThreads, 10)
+  shared_tile_kernel (int nbr, int bs_rt, const __grid_constant__ TilePlan P, const int *__restrict__ row_ptr,
+                      const int *__restrict__ cols, const T *__restrict__ vals, const T *__restrict__ x,
+                      T *__restrict__ y)
 {
   const int r0 = blockIdx.x * P.rows;
   const int nr = min (nbr - r0, P.rows);
   const int B0 = __ldg (row_ptr + r0), n = __ldg (row_ptr + r0 + nr) - B0;
-  if constexpr (shares_tiles (BSC))
-    {
-      const int2 w = window ();
-      const int tile = min (w.x + (int) threadIdx.x, w.y - 1);
-      const int a0 = __ldg (row_ptr + tile * P.rows), a1 = __ldg (row_ptr + min (nbr, (tile + 1) * P.rows));
-      if (n <= kFullTile * P.cap)
-        tile_pass<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y, r0, nr, B0, n);
-      if (__syncthreads_or (a1 - a0 > kFullTile * P.cap))
-        full_tiles<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y);
-    }
-  else
+  const int2 w = window ();
+  const int tile = min (w.x + (int) threadIdx.x, w.y - 1);
+  const int a0 = __ldg (row_ptr + tile * P.rows), a1 = __ldg (row_ptr + min (nbr, (tile + 1) * P.rows));
+  if (n <= kFullTile * P.cap)
     tile_pass<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y, r0, nr, B0, n);
+  if (__syncthreads_or (a1 - a0 > kFullTile * P.cap))
+    full_tiles<T, BSC, V, PAD> (nbr, bs_rt, P, row_ptr, cols, vals, x, y);
 }
 
 template <typename T, int BSC, int V>
@@ -395,7 +406,10 @@ int launch (int nbr, int bs, TilePlan P, const int *rp, const int *c, const T *v
   P.o_first = P.o_rp + up ((P.rows + 1) * 4);
   P.smem = P.o_first + up ((size_t) (P.cap + P.chunk - 1) / P.chunk * 4);
   const unsigned grid = (unsigned) ((nbr + P.rows - 1) / P.rows);
-  tile_kernel<T, BSC, V, PAD><<<grid, kThreads, P.smem, s>>> (nbr, bs, P, rp, c, v, x, y);
+  if constexpr (shares_tiles (BSC))
+    shared_tile_kernel<T, BSC, V, PAD><<<grid, kThreads, P.smem, s>>> (nbr, bs, P, rp, c, v, x, y);
+  else
+    tile_kernel<T, BSC, V, PAD><<<grid, kThreads, P.smem, s>>> (nbr, bs, P, rp, c, v, x, y);
   BMFP_LAUNCH_CHECK ();
   return BMFP_SUCCESS;
 }

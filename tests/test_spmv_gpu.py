@@ -302,9 +302,9 @@ def test_misaligned_arrays_where_aligned_ones_are_staged(lib, orc, cuda, bs, whi
 @pytest.mark.parametrize("bs", [3, 5])
 def test_row_tiles_share_long_rows_that_lie_together(lib, orc, cuda, bs, where, dtype):
     """Tiles that hold many times what a CTA stages, at the ends of the matrix, on
-    both sides of a window's edge and all over: every row right; and not much
-    longer than with the same rows spread (one CTA took them one after the
-    other, six times as long)."""
+    both sides of a window's edge and all over: every row right; and at bs 3,
+    where the tiles are shared, not much longer than with the same rows spread (one
+    CTA took them one after the other, six times as long)."""
     import torch
     rng = np.random.default_rng(bs)
     n, long_rows, length = 60000, 48, 600
@@ -342,7 +342,7 @@ def test_row_tiles_share_long_rows_that_lie_together(lib, orc, cuda, bs, where, 
         crp, cc, cv = orc.bcsr_to_csr(rp, c, v, bs)
         tol = spmv_tolerance(orc, crp, cc, cv, x, dtype)
         assert np.all(np.abs(y[:n * bs] - orc.bcsr_spmv(rp, c, v, bs, x)) <= tol)
-    if where != "everywhere":
+    if bs == 3 and where != "everywhere":
         assert times[where] < 2.5 * times["spread"], times
 
 
